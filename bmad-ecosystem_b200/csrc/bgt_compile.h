@@ -346,6 +346,46 @@ static void put_edge(double* E, const bgt_element& e, bool entering) {
   E[EDGE_GTGS2_2K1] = gt * gs2 - 2 * k1_tane;
 }
 
+// Whether a bend's record is the exact sector body in one step, aligned,
+// without multipoles, with no edge but Hwang's with its constants other than
+// gs2 and g + gt2 zero, and inside the ranges of bend_near (bgt_near.cuh).
+static bool bend_is_plain(const double* q, int32_t flags, int ix, int ixe, int n_step) {
+  if (ix > -1 || ixe > -1 || n_step != 1) return false;
+  if (flags & (F_MISALIGN | F_K1_BODY | F_DRIFT_BODY)) return false;
+  if (flags & (F_EDGE_IN | F_EDGE_OUT)) {
+    for (int end = 0; end < 2; end++) {
+      const double* E = q + B_EDGE + end * EDGE_N;
+      if (!(flags & (end == 0 ? F_EDGE_IN : F_EDGE_OUT))) continue;
+      for (int k : {EDGE_GT, EDGE_GT2, EDGE_K1TANE, EDGE_K1TANE2, EDGE_FG, EDGE_C1, EDGE_C3, EDGE_C4, EDGE_GTGS2_2K1})
+        if (E[k] != 0) return false;
+    }
+  }
+  return q[B_G] != 0 && fabs(q[B_ANGLE]) < 0x1p-4 && q[B_STEP] > 0x1p-20 && q[B_STEP] < 0x1p20 && q[B_BETAREF] > 0.01;
+}
+
+// Whether a compiled record has a near-axis form (F_NEAR)
+static bool record_has_near(const double* rec, const RecHdr& h) {
+  const int32_t fl = h.flags;
+  if (fl & (F_FRINGE_INFO | F_ELEC | F_AP_OFFSET | F_BEND_MIS | F_SOFT_EDGE | F_LINEAR_EDGE | F_NO_HWANG |
+            F_EXACT_EDGE | F_AP_MOMENTUM | F_PITCH | F_HV_KICK))
+    return false;
+  const double* mis = rec + HDR_DW;
+  const double* q = mis + ((fl & F_MISALIGN) ? MIS_N : 0) + ((fl & (F_AP_ENTRANCE | F_AP_EXIT)) ? AP_N : 0);
+  switch (h.kind) {
+    case K_DRIFT:
+      return !(fl & F_MISALIGN);
+    case K_BEND:
+      return bend_is_plain(q, fl, h.ix_mag_max, h.aux1, h.n_step);
+    case K_QUAD:
+    case K_THICK_MULT:
+      // no drift between the nominal edge and the body
+      if ((fl & F_OFFSET) && !(fabs(mis[MIS_DS_SET]) <= 1e-14 && fabs(mis[MIS_DS_UNSET]) <= 1e-14)) return false;
+      return h.aux1 == -1 && h.ix_mag_max <= 7;
+    default:
+      return false;
+  }
+}
+
 // Compile one element into a record.  Returns 0 or BGT_EUNSUPPORTED with err set.
 static int compile_element(const bgt_element& e, const bgt_species& sp, double p0c, std::vector<double>& out,
                            std::string& err) {
@@ -536,7 +576,6 @@ static int compile_element(const bgt_element& e, const bgt_species& sp, double p
 
   RecHdr h{};
   h.kind = kind;
-  h.ix_ele = e.ix_ele;
   h.ix_mag_max = -1;
   h.n_step = 0;
   double an[BGT_N_POLE], bn[BGT_N_POLE];
@@ -763,6 +802,7 @@ static int compile_element(const bgt_element& e, const bgt_species& sp, double p
     for (int n = 0; n <= ix; n++) {
       q[n] = an[n];
       q[ix + 1 + n] = bn[n];
+      if (an[n] != 0 || bn[n] != 0) h.poles |= 1 << n;
     }
   }
   h.aux1 = -1;
@@ -870,6 +910,7 @@ static int compile_element(const bgt_element& e, const bgt_species& sp, double p
     }
   }
   h.flags = flags;
+  if (record_has_near(out.data(), h)) h.flags |= F_NEAR;
   *B.hdr() = h;
   B.finish();
   return 0;
@@ -937,7 +978,6 @@ static int compile_tables(const bgt_element* eles, int32_t n_ele, int32_t n_vari
       int rc = compile_element(eles[(int64_t)v * n_ele + e], sp, p0c, rec, err);
       if (rc) return rc;
       RecHdr* rh = reinterpret_cast<RecHdr*>(rec.data());
-      rh->ix_ele = 0;  // carried by the sequence instead
       if (record_is_rare(rh)) rare = true;
       if (rh->kind == K_QUAD) {
         // quad-matrix memo class: same (b1, length, step) -> same quad_mat2_calc

@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include "bgt_crmath.cuh"
+#include "bgt_fastmath.cuh"
 #include "bgt_qp.cuh"
 #include "bgt_table.h"
 
@@ -55,11 +56,16 @@ __device__ __forceinline__ void set_time(Part& p, qp::Q t) {
 // t = t + dt, dt a real(rp) step, the sum rounded in real(qp)
 __device__ __forceinline__ void add_time(Part& p, double dt) { set_time(p, qp::add(time_of(p), qp::from_double(dt))); }
 
-// Per-particle memo of the drift's pz-only term (track_a_drift.f90:69,
-// first sqrt_one).  Value-identical: recomputed whenever pz differs.
+// Per-particle memo of what depends on pz alone: the drift's pz-only term a
+// (track_a_drift.f90:69, first sqrt_one), r_pc = RN(1 / (1 + pz)), and
+// near_p, the bound on the high words of |px| and |py| below which the
+// near-axis maps hold (0: never, for |pz| >= 2^-3 or beta <= 0).
+// Value-identical: recomputed whenever pz differs.
 struct DriftMemo {
   double pz;
   double a;
+  double r_pc;
+  int32_t near_p;
 };
 
 // Out-of-line device functions (a plain static function in a host build);
@@ -187,7 +193,18 @@ BGT_DEV_NOINLINE XY bend_aperture_frame(Part p, const double* bma, bool at_exit)
 }
 
 // bmad/low_level/orbit_too_large.f90:26-120
+//
+// Nearly every particle is far inside every limit, which the high words show
+// with integer instructions alone: |x|, |y| below max_aperture_limit (the
+// union of two words is at least each of them), and |px|, |py| < 2^-7 with
+// |pz| < 2^-3 leave px^2 + py^2 far below (1 + pz)^2.  Everything else --
+// NaN, a limit that is zero or negative, a particle that may be lost -- takes
+// the comparisons below.  The comparisons alone are 11 FP64 instructions and
+// five branches per element.
 __device__ __forceinline__ bool orbit_too_large(Part& p, const Glob& G) {
+  if (((hi_word(p.x) | hi_word(p.y)) & 0x7fffffff) < hi_word(G.mal) && abs_hi(p.px) < NEAR_P_HI &&
+      abs_hi(p.py) < NEAR_P_HI && abs_hi(p.pz) < NEAR_PZ_HI)
+    return false;
   if (p.x > G.mal) {
     p.state = LOST_POS_X;
     return true;
@@ -363,14 +380,15 @@ __device__ __forceinline__ void check_aperture(Part& p, const double* ap, const 
 // ---------------------------------------------------------------------------
 // Drift: bmad/low_level/track_a_drift.f90:25-116
 
-__device__ __forceinline__ double drift_pz_term(const Part& p, const Glob& G, DriftMemo& m) {
+__device__ __forceinline__ void drift_memo(const Part& p, const Glob& G, DriftMemo& m) {
   if (p.pz != m.pz) {
     double delta = p.pz;
     double rel_pc = 1 + delta;
     m.a = sqrt_one((G.mc2sq * (2 * delta + delta * delta)) / (sq(G.p0c * rel_pc) + G.mc2sq));
+    m.r_pc = 1.0 / rel_pc;
+    m.near_p = (abs_hi(delta) < NEAR_PZ_HI && p.beta > 0) ? NEAR_P_HI : 0;
     m.pz = p.pz;
   }
-  return m.a;
 }
 
 // a / b correctly rounded from r = RN(1 / b): q = RN(a r), e = RN(a - b q)
@@ -419,10 +437,10 @@ __device__ __forceinline__ void track_a_drift(Part& p, double length, const Glob
   double dz;
   if (p.beta > 0) {
     if (REF_MOTION) {
-      double a = drift_pz_term(p, G, m);
+      drift_memo(p, G, m);
       // sqrt_one(-pxy2) = -pxy2 / (sqrt(1 + (-pxy2)) + 1), and
       // sqrt(1 + (-pxy2)) is ps_rel bit for bit (1 + (-a) == 1 - a)
-      dz = length * (a + div_by(-pxy2 / (ps_rel + 1.0), ps_rel, r_ps));
+      dz = length * (m.a + div_by(-pxy2 / (ps_rel + 1.0), ps_rel, r_ps));
     } else {
       dz = -div_by(length, ps_rel, r_ps);
     }

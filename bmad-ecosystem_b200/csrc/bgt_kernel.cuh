@@ -13,6 +13,9 @@
 // block prefix sum through shared memory) so dead lanes stop costing issue
 // slots; fully dead warps skip the element loop.
 //
+// An element's map is its near-axis form where the particle allows it
+// (bgt_near.cuh), else the general map, out of line.
+//
 // Everything up to track1_rec is per-particle arithmetic with no CUDA
 // construct beyond the __device__ qualifiers; a plain C++ compiler that
 // defines those away compiles it for the host (the tests run the element
@@ -669,21 +672,46 @@ __device__ __forceinline__ void body_bend(Part& p, const Rec& R, const Glob& G, 
   element_exit_time(p, t0, z0, q[B_DTREF], G);
 }
 
+}  // namespace bgt
+
+#include "bgt_near.cuh"
+
+namespace bgt {
+
 // track1, bmad/code/track1.f90:43-342 for one alive particle and one record:
 // entrance aperture, body, orbit_too_large, exit aperture.  Returns the
-// particle's state (ALIVE or a lost code).
+// particle with its state (ALIVE or a lost code).  Out of line: in a ring
+// only the RF cavity and the particles near a limit come here, and inlined
+// it would put its code and its register demand into the element loop.  The
+// memo of pz is its own (the caller's stays valid by its key).
+// exit_only: the body is done (by its near-axis form).  The particle goes
+// through memory: passed and returned by value it would tie the element
+// loop's registers to the calling convention.
+struct GeneralCall {
+  Part p;
+  Glob G;
+};
 template <bool RARE>
-__device__ __forceinline__ void track1_rec(Part& p, const double* rec, const Glob& G, DriftMemo& m, QMemo qm) {
+BGT_DEV_NOINLINE void track1_general(GeneralCall* io, const double* rec, QMemo qm, bool exit_only) {
+  Part p = io->p;
+  const Glob G = io->G;
+  struct Store {
+    GeneralCall* io;
+    const Part& p;
+    __device__ __forceinline__ ~Store() { io->p = p; }
+  } store{io, p};
+  DriftMemo m;
+  m.pz = NAN;
   Rec R = decode<RARE>(rec);
   const int32_t fl = R.h->flags;
-  if ((fl & F_AP_ENTRANCE) && G.ap_on) {
+  if (!exit_only && (fl & F_AP_ENTRANCE) && G.ap_on) {
     if (RARE)
       check_aperture(p, R.ap, R.mis, fl, false);
     else
       aperture_limits(p, R.ap, fl, p.x, p.y);
     if (p.state != ALIVE) return;
   }
-  switch (R.h->kind) {
+  switch (exit_only ? (int32_t)K_MARKER : R.h->kind) {
     case K_DRIFT:
       track_a_drift<true>(p, R.kb[DR_L], G, m);
       break;
@@ -712,6 +740,20 @@ __device__ __forceinline__ void track1_rec(Part& p, const double* rec, const Glo
       check_aperture(p, R.ap, R.mis, fl, true);
     else
       aperture_limits(p, R.ap, fl, p.x, p.y);
+  }
+}
+
+template <bool RARE>
+__device__ __forceinline__ void track1_rec(Part& p, const double* rec, const Glob& G, DriftMemo& m, QMemo qm) {
+  const int todo = track1_near<RARE>(p, rec, G, m, qm);
+  if (todo == TODO_NOTHING) return;
+  GeneralCall io = {p, G};
+  track1_general<RARE>(&io, rec, qm, todo == TODO_EXIT);
+  const uint64_t t_lo = p.t_lo, t_hi = p.t_hi;
+  p = io.p;
+  if (!RARE) {  // no particle time in these instances
+    p.t_lo = t_lo;
+    p.t_hi = t_hi;
   }
 }
 
@@ -896,7 +938,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) track_kernel(KArgs a) {
       }
       DriftMemo memo;
       memo.pz = NAN;
-      memo.a = 0;
 #pragma unroll
       for (int c = 0; c < QMEMO_CLASSES; c++) qmemo.q[(c * 13 + 12) * qmemo.stride] = NAN;
       if (p.state == ALIVE && orbit_too_large(p, G)) {
@@ -906,16 +947,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) track_kernel(KArgs a) {
       for (int t = 0; t < a.n_turns; t++) {
         if (__all_sync(0xffffffffu, p.state != ALIVE)) break;  // whole warp lost
         const int turn = a.turn0 + t;
-        for (int r = a.rec_begin; r < a.rec_end; r++) {
-          const int2 e = wseq[r];
-          if (p.state == ALIVE) {
+        if (p.state == ALIVE) {
+          for (int r = a.rec_begin; r < a.rec_end; r++) {
+            const int2 e = wseq[r];
             track1_rec<RARE>(p, wtable + e.x, G, memo, qmemo);
             if (p.state != ALIVE) {
               ixe = e.y;
               ixt = turn;
+              break;
             }
           }
         }
+        __syncwarp();
       }
       if (pidx >= 0) {
         a.vec6[0 * a.n_stride + pidx] = p.x;
@@ -995,7 +1038,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) track_kernel(KArgs a) {
     }
     DriftMemo memo;
     memo.pz = NAN;
-    memo.a = 0;
 #pragma unroll
     for (int c = 0; c < QMEMO_CLASSES; c++) qmemo.q[(c * 13 + 12) * qmemo.stride] = NAN;
     int32_t my_idx = (int32_t)pidx;  // particle carried by this lane (changes on compaction)
@@ -1015,16 +1057,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) track_kernel(KArgs a) {
         // whole warp dead: nothing to do this turn (no block barrier inside
         // the turn unless compaction is on)
       } else {
-        for (int r = a.rec_begin; r < a.rec_end; r++) {
-          const int2 e = seq[r];
-          if (p.state == ALIVE) {
+        if (p.state == ALIVE) {
+          for (int r = a.rec_begin; r < a.rec_end; r++) {
+            const int2 e = seq[r];
             track1_rec<RARE>(p, table + e.x, G, memo, qmemo);
             if (p.state != ALIVE) {
               ixe = e.y;
               ixt = turn;
+              break;
             }
           }
         }
+        __syncwarp();
       }
       // ---- intra-tile compaction (warp ballot + block prefix sum) ----
       if (a.compact_every > 0 && ((t + 1) % a.compact_every) == 0 && t + 1 < a.n_turns) {

@@ -85,16 +85,20 @@ enum Flag : int32_t {
   // F_AP_MOM_ELL: the ecollimator's elliptical pairs
   F_AP_MOMENTUM = 1 << 28,
   F_AP_MOM_ELL = 1 << 29,
+  // the record has a near-axis form (bgt_near.cuh): a drift; a plain bend; a
+  // quadrupole or thick multipole with magnetic multipoles up to order 7 and
+  // offsets and roll at most; lab-frame apertures without momentum limits
+  F_NEAR = 1 << 30,
 };
 
-struct RecHdr {
+struct alignas(8) RecHdr {
   int32_t kind;
-  int32_t ix_ele;
+  int32_t poles;      // bit n: a nonzero multipole a_n or b_n (n <= ix_mag_max)
   int32_t size_dw;    // record size in doubles, header included
   int32_t flags;
   int32_t n_step;     // body steps (quad, bend, thick multipole), slices (rf)
   int32_t ix_mag_max; // highest multipole order with a kick (-1 = none)
-  int32_t aux0;       // kind-specific
+  int32_t aux0;       // quadrupole: matrix memo class
   int32_t aux1;       // kind-specific
 };
 static_assert(sizeof(RecHdr) == 32, "header is 4 doubles");

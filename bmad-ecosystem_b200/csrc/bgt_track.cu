@@ -1095,7 +1095,6 @@ extern "C" int bgt_track_turns_device_noalloc(const bgt_element* eles, int32_t n
     int rc = bgt::host::compile_element(eles[e], *species, p0c, rec, msg);
     if (rc) return fail(rc, msg);
     bgt::RecHdr* rh = reinterpret_cast<bgt::RecHdr*>(rec.data());
-    rh->ix_ele = 0;
     if (bgt::host::record_is_rare(rh)) rare = true;
     if (rh->kind == bgt::K_QUAD) rh->aux0 = -1;  // no quad memo classes on this path
     std::string key(reinterpret_cast<const char*>(rec.data()), rec.size() * sizeof(double));
