@@ -18,7 +18,7 @@ HERE = Path(__file__).resolve().parent
 SRCS = [HERE / "csrc" / "bgt_track.cu", HERE / "csrc" / "bgt_mlp.cu"]
 # the tracking kernel's instances, one compilation per group (bgt_track_kernels.cu)
 KERNEL_SRC = HERE / "csrc" / "bgt_track_kernels.cu"
-N_KERNEL_GROUPS = 10
+N_KERNEL_GROUPS = 12
 OUT = HERE / "bgt" / "libbgt.so"
 
 

@@ -21,8 +21,8 @@ namespace bgt {
 
 // |x|, |y| below max_aperture_limit and |px|, |py| < 2^-7: with |pz| < 2^-3
 // orbit_too_large finds nothing (bgt_device.cuh)
-__device__ __forceinline__ bool inside_limits(double x, double px, double y, double py, const Glob& G) {
-  return ((hi_word(x) | hi_word(y)) & 0x7fffffff) < hi_word(G.mal) && abs_hi(px) < NEAR_P_HI &&
+__device__ __forceinline__ bool inside_limits(double x, double px, double y, double py, double mal) {
+  return ((hi_word(x) | hi_word(y)) & 0x7fffffff) < hi_word(mal) && abs_hi(px) < NEAR_P_HI &&
          abs_hi(py) < NEAR_P_HI;
 }
 
@@ -41,15 +41,15 @@ __device__ __forceinline__ bool inside_aperture(const Part& c, const double* ap,
 
 // track_a_drift for |px|, |py| < 2^-7, |pz| < 2^-3, beta > 0: about 45 FP64
 // instructions and no branch in place of 85 and four range-checked quotients
-// and square roots.  Returns ps_rel.
-__device__ __forceinline__ double drift_near(Part& c, double length, double rel_pc, const DriftMemo& m) {
-  const double px_rel = div_rn(c.px, rel_pc, m.r_pc);
-  const double py_rel = div_rn(c.py, rel_pc, m.r_pc);
+// and square roots.  a and r_pc: the memo of pz.  Returns ps_rel.
+__device__ __forceinline__ double drift_near(Part& c, double length, double rel_pc, double a, double r_pc) {
+  const double px_rel = div_rn(c.px, rel_pc, r_pc);
+  const double py_rel = div_rn(c.py, rel_pc, r_pc);
   const double pxy2 = px_rel * px_rel + py_rel * py_rel;
   const PsTerms T = ps_terms(1 - pxy2);
   c.x = c.x + div_rn(length * px_rel, T.ps, T.r_ps);
   c.y = c.y + div_rn(length * py_rel, T.ps, T.r_ps);
-  c.z = c.z + length * (m.a + div_rn(div_rn(-pxy2, T.ps + 1.0, T.r_ps1), T.ps, T.r_ps));
+  c.z = c.z + length * (a + div_rn(div_rn(-pxy2, T.ps + 1.0, T.r_ps1), T.ps, T.r_ps));
   return T.ps;
 }
 
@@ -81,14 +81,26 @@ struct Saved {
 // ---------------------------------------------------------------------------
 // Magnetic multipole kicks up to order 7 (ab_multipole_kicks).  The factors
 // c_multi(n, m) are signed binomials, here constants of the code (no
-// multiplication by the ones, no look-up); `poles` has bit n set for the
-// orders with a coefficient, so an empty order costs one uniform branch, and
-// a sextupole computes x^2 and y^2 only.  Sums start from their first term:
-// kx_tot and ky_tot start from +0, which absorbs the sign of a zero sum.
+// multiplication by the ones, no look-up).  Sums start from their first
+// term: kx_tot and ky_tot start from +0, which absorbs the sign of a zero
+// sum.
 __device__ __forceinline__ constexpr double binomial(int n, int m) {
   int b = 1;
   for (int i = 1; i <= m; i++) b = b * (n - m + i) / i;
   return b;
+}
+
+// x^k and y^k in mexp's order of products (powi_table7), up to k = TOP
+template <int TOP>
+__device__ __forceinline__ void powers(double x, double (&p)[8]) {
+  p[0] = 1.0;
+  p[1] = x;
+  if (TOP >= 2) p[2] = x * x;
+  if (TOP >= 3) p[3] = x * p[2];
+  if (TOP >= 4) p[4] = p[2] * p[2];
+  if (TOP >= 5) p[5] = x * p[4];
+  if (TOP >= 6) p[6] = p[2] * p[4];
+  if (TOP >= 7) p[7] = p[3] * p[4];
 }
 
 template <int N>
@@ -113,39 +125,69 @@ __device__ __forceinline__ void kick_order(const double (&xp)[8], const double (
   ky_tot = ky_tot + ky;
 }
 
-__device__ __forceinline__ void kicks_near(Part& c, const double* an, const double* bn, int32_t poles, double scale) {
-  double kx = 0, ky = 0;
-  double xp[8], yp[8];
-  xp[0] = yp[0] = 1.0;
-  xp[1] = c.x;
-  yp[1] = c.y;
-  xp[2] = xp[1] * xp[1];
-  yp[2] = yp[1] * yp[1];
-  if (poles & 1) kick_order<0>(xp, yp, scale * an[0], scale * bn[0], kx, ky);
-  if (poles & 2) kick_order<1>(xp, yp, scale * an[1], scale * bn[1], kx, ky);
-  if (poles & 4) kick_order<2>(xp, yp, scale * an[2], scale * bn[2], kx, ky);
-  if (poles >= 8) {
-    // the powers in mexp's order of products (powi_table7)
-    xp[3] = xp[1] * xp[2];
-    yp[3] = yp[1] * yp[2];
-    xp[4] = xp[2] * xp[2];
-    yp[4] = yp[2] * yp[2];
-    xp[5] = xp[1] * xp[4];
-    yp[5] = yp[1] * yp[4];
-    xp[6] = xp[2] * xp[4];
-    yp[6] = yp[2] * yp[4];
+// Orders LO .. HI, all present: one basic block, so that the chains of sums
+// of the orders (N + 1 dependent additions each, 8 cycles apart) overlap: a
+// quadrupole of 16 steps with orders 3 to 6 takes a warp alone on its
+// scheduler 12,900 cycles instead of the 20,500 with a block per order.
+template <int LO, int HI>
+struct DenseKicks {
+  __device__ __forceinline__ static void apply(Part& c, const double* an, const double* bn, int32_t, double scale) {
+    double xp[8], yp[8], kx = 0, ky = 0;
+    powers<HI>(c.x, xp);
+    powers<HI>(c.y, yp);
+    sum(xp, yp, an, bn, scale, kx, ky);
+    c.px = c.px + kx;
+    c.py = c.py + ky;
+  }
+  template <int N = LO>
+  __device__ __forceinline__ static void sum(const double (&xp)[8], const double (&yp)[8], const double* an,
+                                             const double* bn, double scale, double& kx, double& ky) {
+    kick_order<N>(xp, yp, scale * an[N], scale * bn[N], kx, ky);
+    if constexpr (N < HI) sum<N + 1>(xp, yp, an, bn, scale, kx, ky);
+  }
+};
+// Any orders up to 7: one block per order that is present (bit n of poles)
+struct SparseKicks {
+  __device__ __forceinline__ static void apply(Part& c, const double* an, const double* bn, int32_t poles,
+                                               double scale) {
+    double xp[8], yp[8], kx = 0, ky = 0;
+    powers<7>(c.x, xp);
+    powers<7>(c.y, yp);
+    if (poles & 1) kick_order<0>(xp, yp, scale * an[0], scale * bn[0], kx, ky);
+    if (poles & 2) kick_order<1>(xp, yp, scale * an[1], scale * bn[1], kx, ky);
+    if (poles & 4) kick_order<2>(xp, yp, scale * an[2], scale * bn[2], kx, ky);
     if (poles & 8) kick_order<3>(xp, yp, scale * an[3], scale * bn[3], kx, ky);
     if (poles & 16) kick_order<4>(xp, yp, scale * an[4], scale * bn[4], kx, ky);
     if (poles & 32) kick_order<5>(xp, yp, scale * an[5], scale * bn[5], kx, ky);
     if (poles & 64) kick_order<6>(xp, yp, scale * an[6], scale * bn[6], kx, ky);
-    if (poles & 128) {
-      xp[7] = xp[3] * xp[4];
-      yp[7] = yp[3] * yp[4];
-      kick_order<7>(xp, yp, scale * an[7], scale * bn[7], kx, ky);
-    }
+    if (poles & 128) kick_order<7>(xp, yp, scale * an[7], scale * bn[7], kx, ky);
+    c.px = c.px + kx;
+    c.py = c.py + ky;
   }
-  c.px = c.px + kx;
-  c.py = c.py + ky;
+};
+struct NoKicks {
+  __device__ __forceinline__ static void apply(Part&, const double*, const double*, int32_t, double) {}
+};
+
+// f(kicks) for the orders of `poles`: none, dense from the sextupole or the
+// octupole up, else sparse
+template <class F>
+__device__ __forceinline__ bool with_kicks(int32_t poles, const F& f) {
+  switch (poles) {
+    case 0x00: return f(NoKicks{});
+    case 0x04: return f(DenseKicks<2, 2>{});
+    case 0x0c: return f(DenseKicks<2, 3>{});
+    case 0x1c: return f(DenseKicks<2, 4>{});
+    case 0x3c: return f(DenseKicks<2, 5>{});
+    case 0x7c: return f(DenseKicks<2, 6>{});
+    case 0xfc: return f(DenseKicks<2, 7>{});
+    case 0x08: return f(DenseKicks<3, 3>{});
+    case 0x18: return f(DenseKicks<3, 4>{});
+    case 0x38: return f(DenseKicks<3, 5>{});
+    case 0x78: return f(DenseKicks<3, 6>{});
+    case 0xf8: return f(DenseKicks<3, 7>{});
+    default: return f(SparseKicks{});
+  }
 }
 
 // offset_particle without pitch or a drift to the edge (F_NEAR records): the
@@ -176,52 +218,21 @@ __device__ __forceinline__ void offset_near(Part& c, const double* mis, int32_t 
 // ---------------------------------------------------------------------------
 // Quadrupole
 
-// The two quad_mat2_calc results of a body step (once a turn per memo class,
-// or per quadrupole without one): out of line, so that its sine, hyperbolic
-// and quotient code stays out of the element loop.
+// the two quad_mat2_calc results of a body step
 struct QuadMats {
   QMat x, y;
 };
-BGT_DEV_NOINLINE QuadMats quad_mats(double b1, double length, double step, double rel_p) {
-  const double k1 = b1 / (length * rel_p);
-  return {quad_mat2_calc(-k1, step, rel_p), quad_mat2_calc(k1, step, rel_p)};
-}
 
-// body_quad; false, with c unchanged, where low_energy_z_correction takes its
-// exact form, or where a misaligned quadrupole's body leaves the near-axis
-// region.  The correction of a step depends on pz and the element
-// only, so it is evaluated once for all steps.
-__device__ __forceinline__ bool quad_near(Part& c, const RecHdr* h, const double* mis, const double* q, QMemo qm) {
-  const double pz = c.pz;
-  const double* lez = q + Q_LEZ;
-  const double beta0 = lez[LEZ_BETA0];
-  if (!(lez[LEZ_MASS] * ((beta0 * pz) * (beta0 * pz)) < lez[LEZ_3E7])) return false;
-  const double step = q[Q_STEP];
-  const double dz_low = step * pz * (1 - 3 * (pz * (beta0 * beta0)) / 2 + (pz * pz) * lez[LEZ_F]) * lez[LEZ_ME2];
-  const double rel_p = 1 + pz;
-  const int cls = h->aux0, n_step = h->n_step;
-  double* k = qm.q + (cls * 13) * qm.stride;
-  QuadMats M;
-  if (cls >= 0 && k[12 * qm.stride] == rel_p) {
-    const int s = qm.stride;
-    M.x = {k[0], k[s], k[2 * s], k[3 * s], k[4 * s], k[5 * s]};
-    M.y = {k[6 * s], k[7 * s], k[8 * s], k[9 * s], k[10 * s], k[11 * s]};
-  } else {
-    M = quad_mats(q[Q_B1], q[Q_LEN], step, rel_p);
-    if (cls >= 0) {
-      const double v[13] = {M.x.cx, M.x.m01, M.x.m10, M.x.z0, M.x.z1, M.x.z2, M.y.cx,
-                            M.y.m01, M.y.m10, M.y.z0, M.y.z1, M.y.z2, rel_p};
-#pragma unroll
-      for (int j = 0; j < 13; j++) k[j * qm.stride] = v[j];
-    }
-  }
-  const int ix = h->ix_mag_max;
+// The body steps with their kicks
+template <class KICKS>
+__device__ __forceinline__ void quad_steps(Part& c, const QuadMats& M, double dz_low, const RecHdr* h,
+                                           const double* q) {
+  const int n_step = h->n_step;
   const int32_t poles = h->poles;
   const double* an = q + Q_N;
-  const double* bn = an + (ix + 1);
-  Saved start(c);
-  if (h->flags & F_MISALIGN) offset_near(c, mis, h->flags, true);
-  if (ix > -1) kicks_near(c, an, bn, poles, q[Q_RHALF]);
+  const double* bn = an + (h->ix_mag_max + 1);
+  const double r_half = q[Q_RHALF], r_step = q[Q_RSTEP];
+  KICKS::apply(c, an, bn, poles, r_half);
   for (int i = 1; i <= n_step; i++) {
     const double x = c.x, px = c.px, y = c.y, py = c.py;
     c.z = c.z + (M.x.z0 * (x * x) + M.x.z1 * x * px + M.x.z2 * (px * px) + M.y.z0 * (y * y) + M.y.z1 * y * py +
@@ -231,47 +242,95 @@ __device__ __forceinline__ bool quad_near(Part& c, const RecHdr* h, const double
     c.y = M.y.cx * y + M.y.m01 * py;
     c.py = M.y.m10 * y + M.y.cx * py;
     c.z = c.z + dz_low;
-    if (ix > -1) kicks_near(c, an, bn, poles, (i == n_step) ? q[Q_RHALF] : q[Q_RSTEP]);
+    KICKS::apply(c, an, bn, poles, i == n_step ? r_half : r_step);
   }
-  if (h->flags & F_MISALIGN) {
-    // (offset_particle leaves the position of a particle past the momentum
-    // limit as it is)
-    if (!(abs_hi(c.px) < NEAR_P_HI && abs_hi(c.py) < NEAR_P_HI)) {
-      start.restore(c);
-      return false;
-    }
-    offset_near(c, mis, h->flags, false);
+}
+
+// low_energy_z_correction of a step: it depends on pz and the element only,
+// so one value serves all steps.  false where it takes its exact form.
+__device__ __forceinline__ bool quad_low_energy(double pz, const double* q, double& dz_low) {
+  const double* lez = q + Q_LEZ;
+  const double beta0 = lez[LEZ_BETA0];
+  if (!(lez[LEZ_MASS] * ((beta0 * pz) * (beta0 * pz)) < lez[LEZ_3E7])) return false;
+  dz_low = q[Q_STEP] * pz * (1 - 3 * (pz * (beta0 * beta0)) / 2 + (pz * pz) * lez[LEZ_F]) * lez[LEZ_ME2];
+  return true;
+}
+
+// The step matrices from the memo of the element's class; false where it has
+// none for this momentum
+__device__ __forceinline__ bool quad_memo(double rel_p, int cls, QMemo qm, QuadMats& M) {
+  const int s = qm.stride;
+  const double* k = qm.q + (cls * 13) * s;
+  if (!(cls >= 0 && k[12 * s] == rel_p)) return false;
+  M.x = {k[0], k[s], k[2 * s], k[3 * s], k[4 * s], k[5 * s]};
+  M.y = {k[6 * s], k[7 * s], k[8 * s], k[9 * s], k[10 * s], k[11 * s]};
+  return true;
+}
+__device__ __forceinline__ void quad_memo_fill(double rel_p, int cls, QMemo qm, const double* q, QuadMats& M) {
+  const double k1 = q[Q_B1] / (q[Q_LEN] * rel_p);
+  M = {quad_mat2_calc(-k1, q[Q_STEP], rel_p), quad_mat2_calc(k1, q[Q_STEP], rel_p)};
+  if (cls < 0) return;
+  double* k = qm.q + (cls * 13) * qm.stride;
+  const double v[13] = {M.x.cx, M.x.m01, M.x.m10, M.x.z0, M.x.z1, M.x.z2, M.y.cx,
+                        M.y.m01, M.y.m10, M.y.z0, M.y.z1, M.y.z2, rel_p};
+#pragma unroll
+  for (int j = 0; j < 13; j++) k[j * qm.stride] = v[j];
+}
+
+// ---------------------------------------------------------------------------
+// Thick multipole: kick, drift, ..., kick; false when a kick leaves the
+// near-axis region before a drift
+template <class KICKS>
+__device__ __forceinline__ bool thick_steps(Part& c, const RecHdr* h, const double* q, double mal, double a,
+                                            double r_pc) {
+  const int n_step = h->n_step;
+  const int32_t poles = h->poles;
+  const double* an = q + TM_N;
+  const double* bn = an + (h->ix_mag_max + 1);
+  const double step = q[TM_STEP], rel_pc = 1 + c.pz;
+  const double r_half = q[TM_RHALF], r_step = q[TM_RSTEP];
+  KICKS::apply(c, an, bn, poles, r_half);
+  for (int i = 1; i <= n_step; i++) {
+    if (!inside_limits(c.x, c.px, c.y, c.py, mal)) return false;
+    if (step != 0) drift_near(c, step, rel_pc, a, r_pc);
+    KICKS::apply(c, an, bn, poles, i == n_step ? r_half : r_step);
   }
   return true;
 }
 
-// body_thick: kick, drift, ..., kick; false, with c unchanged, when a kick
-// leaves the near-axis region before a drift or the exit offset
-__device__ __forceinline__ bool thick_near(Part& c, const RecHdr* h, const double* mis, const double* q,
-                                           const Glob& G, const DriftMemo& m) {
-  const int32_t fl = h->flags, poles = h->poles;
-  const int ix = h->ix_mag_max, n_step = h->n_step;
-  const double* an = q + TM_N;
-  const double* bn = an + (ix + 1);
-  const double step = q[TM_STEP], rel_pc = 1 + c.pz;
-  Saved start(c);
+// ---------------------------------------------------------------------------
+// The body of any F_NEAR quadrupole or thick multipole.  Called out of line
+// (track1_general) for the ones that are misaligned or carry multipoles other
+// than a sextupole's, and where a quadrupole's matrices are not in the memo,
+// so that the element loop holds the registers and the code of the plain ones
+// only; the call costs ~280 instructions, of 950 for a sextupole and 3800 for
+// a quadrupole of 16 steps (inlined, they raised every drift's spills from 6
+// loads to 13).  false, p unchanged, for the general maps: the exact
+// low-energy correction, or a particle that leaves the near-axis region on
+// the way (offset_particle then leaves its position as it is).
+__device__ __forceinline__ bool body_near(Part& p, const RecHdr* h, const double* mis, const double* q, double mal,
+                                          double a, double r_pc, QMemo qm) {
+  Part c = p;
+  const int32_t fl = h->flags;
   if (fl & F_MISALIGN) offset_near(c, mis, fl, true);
-  if (ix > -1) kicks_near(c, an, bn, poles, q[TM_RHALF]);
-  for (int i = 1; i <= n_step; i++) {
-    if (!inside_limits(c.x, c.px, c.y, c.py, G)) {
-      start.restore(c);
+  if (h->kind == K_QUAD) {
+    QuadMats M;
+    double dz_low;
+    if (!quad_low_energy(c.pz, q, dz_low)) return false;
+    if (!quad_memo(1 + c.pz, h->aux0, qm, M)) quad_memo_fill(1 + c.pz, h->aux0, qm, q, M);
+    with_kicks(h->poles, [&](auto kicks) {
+      quad_steps<decltype(kicks)>(c, M, dz_low, h, q);
+      return true;
+    });
+  } else {
+    if (!with_kicks(h->poles, [&](auto kicks) { return thick_steps<decltype(kicks)>(c, h, q, mal, a, r_pc); }))
       return false;
-    }
-    if (step != 0) drift_near(c, step, rel_pc, m);
-    if (ix > -1) kicks_near(c, an, bn, poles, (i == n_step) ? q[TM_RHALF] : q[TM_RSTEP]);
   }
   if (fl & F_MISALIGN) {
-    if (!(abs_hi(c.px) < NEAR_P_HI && abs_hi(c.py) < NEAR_P_HI)) {
-      start.restore(c);
-      return false;
-    }
+    if (!(abs_hi(c.px) < NEAR_P_HI && abs_hi(c.py) < NEAR_P_HI)) return false;
     offset_near(c, mis, fl, false);
   }
+  p = c;
   return true;
 }
 
@@ -319,7 +378,7 @@ __device__ __forceinline__ bool bend_near(Part& p, const double* q, int32_t fl, 
   const double pz = p.pz;
   const double e = m.r_pc;
   if (fl & F_EDGE_IN) hwang_edge_normal<true>(x, px, y, py, z, e, q + B_EDGE);
-  bad |= !inside_limits(x, px, y, py, G);
+  bad |= !inside_limits(x, px, y, py, G.mal);
   // the semi-linear map needs |px|, |py|, |pz| < 1e-9 (high word 0x3e112e0b)
   if (fl & F_SEMI_LINEAR_OK)
     bad |= abs_hi(px) <= 0x3e112e0b && abs_hi(py) <= 0x3e112e0b && abs_hi(pz) <= 0x3e112e0b;
@@ -358,7 +417,7 @@ __device__ __forceinline__ bool bend_near(Part& p, const double* q, int32_t fl, 
   const double px1 = pt * odd_small(arg, cr::SIN_C, bad);
   double y1 = y + div_rn(py * L_p, pt, r_pt);
   double z1 = z + div_rn(p.beta * step_len, q[B_BETAREF], q[B_RBETAREF]) - div_rn(rel_p * L_p, pt, r_pt);
-  bad |= !inside_limits(x1, px1, y1, py, G);
+  bad |= !inside_limits(x1, px1, y1, py, G.mal);
   double x2 = x1;
   if (fl & F_EDGE_OUT) hwang_edge_normal<false>(x2, px1, y1, py, z1, e, q + B_EDGE + EDGE_N);
   p.x = x2;
@@ -371,30 +430,30 @@ __device__ __forceinline__ bool bend_near(Part& p, const double* q, int32_t fl, 
 }
 
 // ---------------------------------------------------------------------------
-// track1 through a record by its near-axis form.  What is left to the general
-// maps: TODO_NOTHING; TODO_EXIT, the checks after the body, where the particle
-// may be past a limit or an aperture; TODO_ALL, the whole element, p as it
-// was.  TIME: the instance carries the particle time.
-enum NearTodo : int { TODO_NOTHING = 0, TODO_EXIT = 1, TODO_ALL = 2 };
+// track1 through a record by its near-axis form.  What is left to do out of
+// line (track1_general): TODO_NOTHING; TODO_EXIT, the checks after the body,
+// where the particle may be past a limit or an aperture; TODO_BODY, the body
+// by body_near and those checks; TODO_ALL, the whole element by the general
+// maps.  With the last two p is as it was.  TIME: the instance carries the
+// particle time.
+enum NearTodo : int { TODO_NOTHING = 0, TODO_EXIT = 1, TODO_BODY = 2, TODO_ALL = 3 };
 
 template <bool TIME>
 __device__ __forceinline__ int track1_near(Part& p, const double* rec, const Glob& G, DriftMemo& m, QMemo qm) {
   const RecHdr* h = reinterpret_cast<const RecHdr*>(rec);
-  const int32_t fl = h->flags;
+  const int32_t kind = h->kind, fl = h->flags;
   if (!(fl & F_NEAR)) return TODO_ALL;
   drift_memo(p, G, m);
   if (!(abs_hi(p.px) < m.near_p && abs_hi(p.py) < m.near_p)) return TODO_ALL;
   const double* q = rec + HDR_DW;
-  const double* mis = q;
   if (fl & F_MISALIGN) q += MIS_N;
   const double* ap = q;
   if (fl & (F_AP_ENTRANCE | F_AP_EXIT)) q += AP_N;
   if ((fl & F_AP_ENTRANCE) && G.ap_on && !inside_aperture(p, ap, fl)) return TODO_ALL;
-  const int32_t kind = h->kind;
   if (kind == K_DRIFT) {
     const double length = q[DR_L];
     if (length != 0) {
-      const double ps = drift_near(p, length, 1 + p.pz, m);
+      const double ps = drift_near(p, length, 1 + p.pz, m.a, m.r_pc);
       if (TIME && G.track_time) add_time(p, length / (p.beta * ps * C_LIGHT));
     }
   } else {
@@ -405,15 +464,24 @@ __device__ __forceinline__ int track1_near(Part& p, const double* rec, const Glo
       if (!bend_near(p, q, fl, G, m)) return TODO_ALL;
       dt_ref = q[B_DTREF];
     } else if (kind == K_QUAD) {
-      if (!quad_near(p, h, mis, q, qm)) return TODO_ALL;
+      QuadMats M;
+      double dz_low;
+      if ((fl & F_MISALIGN) || h->poles != 0 || !quad_memo(1 + p.pz, h->aux0, qm, M)) return TODO_BODY;
+      if (!quad_low_energy(p.pz, q, dz_low)) return TODO_ALL;
+      quad_steps<NoKicks>(p, M, dz_low, h, q);
       dt_ref = q[Q_DTREF];
     } else {
-      if (!thick_near(p, h, mis, q, G, m)) return TODO_ALL;
+      if ((fl & F_MISALIGN) || h->poles != 4) return TODO_BODY;
+      Saved start(p);
+      if (!thick_steps<DenseKicks<2, 2>>(p, h, q, G.mal, m.a, m.r_pc)) {
+        start.restore(p);
+        return TODO_ALL;
+      }
       dt_ref = q[TM_DTREF];
     }
     if (TIME) element_exit_time(p, t0, z0, dt_ref, G);
   }
-  if (!inside_limits(p.x, p.px, p.y, p.py, G)) return TODO_EXIT;
+  if (!inside_limits(p.x, p.px, p.y, p.py, G.mal)) return TODO_EXIT;
   if ((fl & F_AP_EXIT) && G.ap_on && !inside_aperture(p, ap, fl)) return TODO_EXIT;
   return TODO_NOTHING;
 }

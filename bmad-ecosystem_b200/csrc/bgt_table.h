@@ -93,13 +93,13 @@ enum Flag : int32_t {
 
 struct alignas(8) RecHdr {
   int32_t kind;
-  int32_t poles;      // bit n: a nonzero multipole a_n or b_n (n <= ix_mag_max)
-  int32_t size_dw;    // record size in doubles, header included
   int32_t flags;
-  int32_t n_step;     // body steps (quad, bend, thick multipole), slices (rf)
+  int32_t poles;      // bit n: a nonzero multipole a_n or b_n (n <= ix_mag_max)
   int32_t ix_mag_max; // highest multipole order with a kick (-1 = none)
+  int32_t n_step;     // body steps (quad, bend, thick multipole), slices (rf)
   int32_t aux0;       // quadrupole: matrix memo class
   int32_t aux1;       // kind-specific
+  int32_t size_dw;    // record size in doubles, header included
 };
 static_assert(sizeof(RecHdr) == 32, "header is 4 doubles");
 

@@ -192,11 +192,13 @@ TrackKernelGroup track_kernel_group_6();
 TrackKernelGroup track_kernel_group_7();
 TrackKernelGroup track_kernel_group_8();
 TrackKernelGroup track_kernel_group_9();
+TrackKernelGroup track_kernel_group_10();
+TrackKernelGroup track_kernel_group_11();
 TrackKernelGroup track_kernel_group(int g) {
   static TrackKernelGroup (*const groups[N_KERNEL_GROUPS])() = {
       track_kernel_group_0, track_kernel_group_1, track_kernel_group_2, track_kernel_group_3,
       track_kernel_group_4, track_kernel_group_5, track_kernel_group_6, track_kernel_group_7,
-      track_kernel_group_8, track_kernel_group_9};
+      track_kernel_group_8, track_kernel_group_9, track_kernel_group_10, track_kernel_group_11};
   return groups[g]();
 }
 }  // namespace bgt

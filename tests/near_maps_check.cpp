@@ -187,18 +187,18 @@ static void one_form(const char* name, bgt_element e, long n) {
     DriftMemo m;
     m.pz = NAN;
     const int todo = track1_near<false>(a, rec, G, m, QMemo{qa, 1});
-    GeneralCall io = {p, G};
-    track1_general<false>(&io, rec, QMemo{qb, 1}, false);
-    if (todo != TODO_NOTHING) {  // what is left to the general maps gives the same
-      GeneralCall rest = {a, G};
-      track1_general<false>(&rest, rec, QMemo{qa, 1}, todo == TODO_EXIT);
+    GeneralCall io = {p, &G, 0, 0};
+    track1_general<false>(&io, rec, QMemo{qb, 1}, TODO_ALL);
+    if (todo != TODO_NOTHING) {  // what is left to do out of line gives the same
+      GeneralCall rest = {a, &G, m.a, m.r_pc};
+      track1_general<false>(&rest, rec, QMemo{qa, 1}, todo);
       a = rest.p;
     }
     const Part& b = io.p;
     const bool equal = same(a.x, b.x) && same(a.px, b.px) && same(a.y, b.y) && same(a.py, b.py) && same(a.z, b.z) &&
                        a.pz == b.pz && a.beta == b.beta && a.state == b.state;
     c.total++;
-    if (todo == TODO_NOTHING) c.passed++;
+    if (todo == TODO_NOTHING || todo == TODO_BODY) c.passed++;
     if (!equal) c.bad++;
   }
 }
