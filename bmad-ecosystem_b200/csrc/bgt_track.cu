@@ -174,8 +174,8 @@ static bgt_tuning get_tuning_locked(bgt_handle* h) {
 // Dynamic shared memory of a launch: the table (unless read from global
 // memory), the compaction stage (9 rows of BLOCK doubles, 11 with the
 // particle times of the RARE instances) and the quadrupole memo.
-static size_t smem_bytes(const bgt_handle* h, int block, bool compact, bool gtab, bool rare) {
-  size_t b = gtab ? 0 : (size_t)h->table_dw * 8;
+static size_t smem_bytes(size_t table_dw, int block, bool compact, bool gtab, bool rare) {
+  size_t b = gtab ? 0 : table_dw * 8;
   if (compact) b += (size_t)(rare ? 11 : 9) * block * 8;
   b += (size_t)QMEMO_CLASSES * 13 * block * 8;
   return b;
@@ -240,17 +240,53 @@ static uint64_t wait_ns_of(const bgt_tuning& t) {
   return t.wait_limit_us > 0 ? (uint64_t)t.wait_limit_us * 1000ull : 2000000000ull;
 }
 
+// A tuning fitted to a call: the shape and table placement to launch.
+// n_tiles(block): the tiles of `block` particles that the call makes.
+//
+// * 256-thread tiles become 128-thread ones with the same register cap while
+//   all of them are resident at once: a CTA's warps share an SM, so few large
+//   tiles leave SMs idle or uneven.  Measured on B200, 256 x 2 against
+//   128 x 4: 40,000 particles x 4 turns of the FODO ring 2.70 / 2.40 ms,
+//   10,000 2.25 / 2.07 ms, one turn of 8,064 probes on four error rings
+//   2.08 / 1.90 ms; from one full wave on they are equal.
+// * table_mode 0 stages the table in shared memory only if that leaves room
+//   for the CTAs the launch can use per SM; a staged 150 KB table (error
+//   rings) holds one.  Staged against global, 128 x 4, one turn on error
+//   rings: 60,000 particles (4 CTAs per SM wanted) 7.39 / 3.31 ms, 32,000 (2)
+//   3.75 / 2.33 ms, 16,000 (1) 1.92 / 2.15 ms.
+template <class NTiles>
+static bgt_tuning fit_tuning(bgt_tuning t, size_t table_dw, int num_sms, bool rare, const NTiles& n_tiles) {
+  const bool compact = t.compact_every > 0;
+  // whether a staged table leaves every CTA resident that the launch can use
+  // (228 KB of shared memory per SM, 1 KB of it per CTA reserved)
+  auto staged_fits = [&](int block, int per_sm) {
+    const size_t smem = smem_bytes(table_dw, block, compact, false, rare);
+    const int64_t wanted = std::min<int64_t>(per_sm, (n_tiles(block) + num_sms - 1) / num_sms);
+    return smem <= SMEM_LIMIT && (int64_t)((228 * 1024) / (smem + 1024)) >= wanted;
+  };
+  const int mode = t.table_mode >= 2 ? t.table_mode - 1 : 0;  // the kernels' TMODE
+  if (t.threads_per_block == 256 && n_tiles(256) < (int64_t)t.blocks_per_sm * num_sms &&
+      find_track_kernel(128, 2 * t.blocks_per_sm, mode, rare) && (mode != 0 || staged_fits(128, 2 * t.blocks_per_sm))) {
+    t.threads_per_block = 128;
+    t.blocks_per_sm *= 2;
+  }
+  if (t.table_mode == 0 && !staged_fits(t.threads_per_block, t.blocks_per_sm) &&
+      find_track_kernel(t.threads_per_block, t.blocks_per_sm, 1, rare))
+    t.table_mode = 2;
+  return t;
+}
+
 // The kernel instance for a tuning and a shared-memory need, with the
 // placement of the table it implies; 0 or an error code.
 static int pick_kernel(bgt_handle* h, const bgt_tuning& tun, bool compact, bool rare, LaunchFn* fn,
                        size_t* smem) {
   const int block = tun.threads_per_block;
-  const bool fits = smem_bytes(h, block, compact, false, rare) <= SMEM_LIMIT;
+  const bool fits = smem_bytes(h->table_dw, block, compact, false, rare) <= SMEM_LIMIT;
   if (tun.table_mode == 1 && !fits)
     return set_err(h, BGT_ETOOLARGE, "element table does not fit in shared memory (table_mode 1)");
   const bool gtab = tun.table_mode >= 2 || !fits;
   const bool warp_sched = tun.table_mode == 3;
-  *smem = smem_bytes(h, block, compact, gtab, rare);
+  *smem = smem_bytes(h->table_dw, block, compact, gtab, rare);
   if (*smem > SMEM_LIMIT) return set_err(h, BGT_ETOOLARGE, "tracking state does not fit in shared memory");
   *fn = find_track_kernel(block, tun.blocks_per_sm, gtab ? (warp_sched ? 2 : 1) : 0, rare);
   if (!*fn) {
@@ -286,6 +322,17 @@ static int enqueue_track(bgt_handle* h, const bgt_tuning& tun, CallCtx* c, KArgs
   if (e != cudaSuccess) return set_err(h, BGT_ECUDA, std::string("track_kernel launch: ") + cudaGetErrorString(e));
   h->launches++;
   return 0;
+}
+
+// The handle's tuning fitted to a call whose particles come in groups, one per
+// lattice variant, of the given sizes.
+static bgt_tuning call_tuning(bgt_handle* h, const bgt_tuning& tun, const std::vector<int64_t>& groups,
+                              bool with_time) {
+  return fit_tuning(tun, (size_t)h->table_dw, h->num_sms, h->rare || with_time, [&](int block) {
+    int64_t tiles = 0;
+    for (int64_t g : groups) tiles += (g + block - 1) / block;
+    return tiles;
+  });
 }
 
 static KArgs base_args(bgt_handle* h, const bgt_tuning& tun) {
@@ -480,20 +527,21 @@ int bgt_track_turns_device(bgt_handle* h, double* d_vec6, double* d_beta, void* 
   if (n > INT32_MAX) return set_err(h, BGT_EINVAL, "bgt_track_turns_device: n exceeds 2^31 - 1");
   DeviceGuard dg(h->device);
   CU(h, dg.err);
-  const bgt_tuning tun = get_tuning_locked(h);
+  bgt_tuning tun = get_tuning_locked(h);
   cudaStream_t st = (cudaStream_t)stream;
   CtxLease L(h);
   int rc = L.acquire();
   if (rc) return rc;
   CallCtx* c = L.c;
   CU(h, L.use(st));
-  if (!d_variant || h->n_variants == 1)
+  if (!d_variant || h->n_variants == 1) {
+    tun = call_tuning(h, tun, {n}, tq != nullptr);
     return track_device_impl(h, tun, c, h->d_status, d_vec6, n, d_beta, tq, d_state, d_ix_ele_lost,
                              d_ix_turn_lost, nullptr, nullptr, n, n, turn0, n_turns, 0, h->n_ele, st);
+  }
   // Group by variant into tile-aligned slot ranges.  The variant ids must be
   // sorted (non-decreasing); the per-variant counts are read back once.
   const int32_t nv = h->n_variants;
-  const int block = tun.threads_per_block;
   if (!c->d_grp_v) CU(h, cudaMalloc(&c->d_grp_v, ((size_t)3 * nv + 1) * 8));
   int64_t* d_first = c->d_grp_v;
   int64_t* d_count = d_first + nv;
@@ -502,13 +550,15 @@ int bgt_track_turns_device(bgt_handle* h, double* d_vec6, double* d_beta, void* 
   CU(h, cudaMemsetAsync(d_first, 0, ((size_t)3 * nv + 1) * 8, st));
   variant_count_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_variant, n, nv, d_first, d_count, d_bad);
   h->launches++;
-  std::vector<int64_t> cnt((size_t)nv + 1);
+  std::vector<int64_t> cnt((size_t)nv);
   CU(h, cudaMemcpyAsync(cnt.data(), d_count, (size_t)nv * 8, cudaMemcpyDeviceToHost, st));
   int32_t bad = 0;
   CU(h, cudaMemcpyAsync(&bad, d_bad, 4, cudaMemcpyDeviceToHost, st));
   CU(h, cudaStreamSynchronize(st));
   if (bad & 1) return set_err(h, BGT_EINVAL, "bgt_track_turns_device: variant id out of range");
   if (bad & 2) return set_err(h, BGT_EINVAL, "bgt_track_turns_device: variant ids must be sorted");
+  tun = call_tuning(h, tun, cnt, tq != nullptr);
+  const int block = tun.threads_per_block;
   std::vector<int64_t> slot0(nv);
   std::vector<int32_t> tvar;
   int64_t s = 0;
@@ -645,8 +695,7 @@ static int track_host(bgt_handle* h, double* vec6, double* beta, void* t, int32_
   if (n > INT32_MAX) return set_err(h, BGT_EINVAL, "n exceeds 2^31 - 1");
   DeviceGuard dg(h->device);
   CU(h, dg.err);
-  const bgt_tuning tun = get_tuning_locked(h);
-  const int block = tun.threads_per_block;
+  bgt_tuning tun = get_tuning_locked(h);
   // group particles by variant into tile-aligned slot ranges
   std::vector<int32_t> slot_map, tile_var;
   int64_t n_slots = n;
@@ -657,6 +706,8 @@ static int track_host(bgt_handle* h, double* vec6, double* beta, void* t, int32_
       if (variant[i] < 0 || variant[i] >= h->n_variants) return set_err(h, BGT_EINVAL, "variant out of range");
       count[variant[i]]++;
     }
+    tun = call_tuning(h, tun, count, t != nullptr);
+    const int block = tun.threads_per_block;
     std::vector<int64_t> start(h->n_variants, 0);
     int64_t s = 0;
     for (int v = 0; v < h->n_variants; v++) {
@@ -673,6 +724,8 @@ static int track_host(bgt_handle* h, double* vec6, double* beta, void* t, int32_
     for (int64_t i = 0; i < n; i++)
       if (variant[i] != 0) return set_err(h, BGT_EINVAL, "variant out of range");
   }
+  if (!multi) tun = call_tuning(h, tun, {n}, t != nullptr);
+  const int block = tun.threads_per_block;
   int64_t n_tiles = (n_slots + block - 1) / block;
   CtxLease L(h);
   int rc = L.acquire();
@@ -877,7 +930,9 @@ int bgt_da_scan_grid(bgt_handle* h, const double* ref_orbit, int32_t n_variants_
     return set_err(h, BGT_EINVAL, "bgt_da_scan_grid: invalid argument");
   DeviceGuard dg(h->device);
   CU(h, dg.err);
-  const bgt_tuning tun = get_tuning_locked(h);
+  const bgt_tuning tun =
+      call_tuning(h, get_tuning_locked(h),
+                  std::vector<int64_t>(n_variants_used, (int64_t)n_delta * n_angle * n_radius), h->G.abs_time != 0);
   const int block = tun.threads_per_block;
   DAArgs A{};
   A.n_var = n_variants_used;
@@ -1119,18 +1174,18 @@ extern "C" int bgt_track_turns_device_noalloc(const bgt_element* eles, int32_t n
     return fail(BGT_ETOOLARGE, "bgt_track_turns_device_noalloc: element table needs " +
                                    std::to_string(table_bytes) + " bytes, the scratch array holds " +
                                    std::to_string(BGT_NOALLOC_SCRATCH_BYTES - 256));
-  // The table is staged in shared memory when it fits, else read in place
-  // from the scratch array (global memory, CTA tiles), as bgt_create's
-  // tables are.
-  const int block = t.threads_per_block;
-  const size_t state_smem = (t.compact_every > 0 ? (size_t)9 * block * 8 : 0) +
-                            (size_t)bgt::QMEMO_CLASSES * 13 * block * 8;
-  const bool gtab = state_smem + table_bytes > SMEM_LIMIT;
-  const size_t smem = state_smem + (gtab ? 0 : table_bytes);
-  const LaunchFn launch = find_track_kernel(block, t.blocks_per_sm, gtab ? 1 : 0, rare);
-  if (!launch) return fail(BGT_EINVAL, "bgt_track_turns_device_noalloc: no kernel instance for this tuning");
+  // The table is staged in shared memory where that is the better place
+  // (fit_tuning), else read in place from the scratch array (global memory,
+  // CTA tiles), as bgt_create's tables are.
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  t.table_mode = 0;
+  t = fit_tuning(t, tab.size(), sms, rare, [n](int block) { return (n + block - 1) / block; });
+  const int block = t.threads_per_block;
+  const bool gtab = t.table_mode != 0 || smem_bytes(tab.size(), block, t.compact_every > 0, false, rare) > SMEM_LIMIT;
+  const size_t smem = smem_bytes(tab.size(), block, t.compact_every > 0, gtab, rare);
+  const LaunchFn launch = find_track_kernel(block, t.blocks_per_sm, gtab ? 1 : 0, rare);
+  if (!launch) return fail(BGT_EINVAL, "bgt_track_turns_device_noalloc: no kernel instance for this tuning");
 
   cudaStream_t st = (cudaStream_t)stream;
   int32_t* d_counter = reinterpret_cast<int32_t*>(base);

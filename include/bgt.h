@@ -177,10 +177,11 @@ typedef struct bgt_tuning {
   int32_t blocks_per_sm;     /* resident CTAs per SM for the persistent grid */
   int32_t turns_per_launch;  /* turns per persistent-kernel launch (graph node) */
   int32_t compact_every;     /* compact lost particles every this many turns (0 = never) */
-  int32_t table_mode;        /* element table: 0 = staged in shared memory when it fits, else read
-                                from global memory; 1 = shared memory only; 2 = global memory;
-                                3 = global memory with every warp scheduled on its own (no
-                                CTA-wide tiles: for small, long-lived particle sets) */
+  int32_t table_mode;        /* element table: 0 = staged in shared memory when it fits beside the
+                                other CTAs the call can use per SM, else read from global memory;
+                                1 = shared memory only; 2 = global memory; 3 = global memory with
+                                every warp scheduled on its own (no CTA-wide tiles: for small,
+                                long-lived particle sets) */
   int32_t wait_limit_us;     /* bound of the kernel's wait for its element-table copy, in
                                 microseconds (0 = 2 s); when it runs out the kernel sets its error
                                 flag and returns: BGT_ETIMEOUT from host-buffer calls, from
