@@ -233,7 +233,9 @@ class SurvivalMLP:
             _need(variant, torch.int32, "variant")
         n = vec.shape[1]
         dev = vec.device
-        x = torch.zeros((pad_rows(n), N_IN), dtype=torch.bfloat16, device=dev) if normalized else None
+        x = torch.empty((pad_rows(n), N_IN), dtype=torch.bfloat16, device=dev) if normalized else None
+        if x is not None and pad_rows(n) != n:
+            x[n:].zero_()  # the library writes the n rows
         r = torch.empty((n, N_FEATURES), dtype=torch.float32, device=dev) if raw else None
         rc = self.lib.bgt_mlp_features(vec0.data_ptr(), vec.data_ptr(), n, vec.shape[1],
                                        variant.data_ptr() if variant is not None else None, table.data_ptr(),

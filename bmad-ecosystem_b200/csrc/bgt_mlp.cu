@@ -759,34 +759,84 @@ __global__ void pack_kernel(const float* __restrict__ p, bf16* __restrict__ w1, 
   }
 }
 
-__global__ void features_kernel(const double* __restrict__ vec0, const double* __restrict__ vec, int64_t n,
-                                int64_t stride, const int32_t* __restrict__ var, const double* __restrict__ table,
-                                const float* __restrict__ mean, const float* __restrict__ inv_std,
-                                float* __restrict__ raw, bf16* __restrict__ x) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double* T = table + (int64_t)(var ? var[i] : 0) * BGT_MLP_VARIANT_COLS;
-  double f[BGT_MLP_FEATURES];
-  for (int k = 0; k < 6; k++) f[k] = vec0[k * stride + i] - T[k];
-  for (int k = 0; k < 16; k++) f[6 + k] = T[14 + k];
-  for (int k = 0; k < 6; k++) f[22 + k] = vec[k * stride + i] - T[k];
-  const double dp = f[27];
-  const double xb = f[22] - T[6] * dp, pxb = f[23] - T[7] * dp;
-  const double yb = f[24] - T[8] * dp, pyb = f[25] - T[9] * dp;
-  const double ba = T[10], aa = T[11], bb = T[12], ab = T[13];
-  const double ja = 0.5 * ((1 + aa * aa) / ba * xb * xb + 2 * aa * xb * pxb + ba * pxb * pxb);
-  const double jb = 0.5 * ((1 + ab * ab) / bb * yb * yb + 2 * ab * yb * pyb + bb * pyb * pyb);
-  f[28] = sqrt(fmax(ja, 0.0));
-  f[29] = sqrt(fmax(jb, 0.0));
-  if (raw)
-    for (int k = 0; k < BGT_MLP_FEATURES; k++) raw[i * BGT_MLP_FEATURES + k] = (float)f[k];
+// Classifier inputs of n particles, one thread each.  Memory-bound: 100 B in,
+// 128 B (x) and 120 B (raw) out per particle.  A thread's row is written to
+// shared memory and the block's rows, which are contiguous, leave it in
+// 16-byte stores by consecutive threads; stored by the thread that owns the
+// row, every store instruction touched 32 lines.  Chunk c of row r sits at c ^
+// (r % 8), free of bank conflicts both ways; raw rows are 31 floats apart.
+// 500,001 particles through the Python call: 60 us (with a zero fill of all of
+// x) -> 31.5 us, 3.6 TB/s.
+constexpr int FEAT_BLOCK = 128;
+__global__ void __launch_bounds__(FEAT_BLOCK)
+    features_kernel(const double* __restrict__ vec0, const double* __restrict__ vec, int64_t n, int64_t stride,
+                    const int32_t* __restrict__ var, const double* __restrict__ table,
+                    const float* __restrict__ mean, const float* __restrict__ inv_std, float* __restrict__ raw,
+                    bf16* __restrict__ x) {
+  extern __shared__ __align__(16) uint8_t feat_smem[];
+  __shared__ float norm_s[2][BGT_MLP_FEATURES];
+  const int tid = threadIdx.x;
+  const int64_t i0 = blockIdx.x * (int64_t)FEAT_BLOCK, i = i0 + tid;
+  const int rows = (int)min((int64_t)FEAT_BLOCK, n - i0);
+  if (x && tid < BGT_MLP_FEATURES) {
+    norm_s[0][tid] = mean[tid];
+    norm_s[1][tid] = inv_std[tid];
+  }
+  uint4* xs = reinterpret_cast<uint4*>(feat_smem);
+  float* rs = reinterpret_cast<float*>(feat_smem + (x ? FEAT_BLOCK * IN * sizeof(bf16) : 0));
+  float f[BGT_MLP_FEATURES];
+  if (i < n) {
+    const double* T = table + (int64_t)(var ? var[i] : 0) * BGT_MLP_VARIANT_COLS;
+    double v[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      f[k] = (float)(vec0[k * stride + i] - T[k]);
+      v[k] = vec[k * stride + i] - T[k];
+      f[22 + k] = (float)v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) f[6 + k] = (float)T[14 + k];
+    const double dp = v[5];
+    const double xb = v[0] - T[6] * dp, pxb = v[1] - T[7] * dp;
+    const double yb = v[2] - T[8] * dp, pyb = v[3] - T[9] * dp;
+    const double ba = T[10], aa = T[11], bb = T[12], ab = T[13];
+    const double ja = 0.5 * ((1 + aa * aa) / ba * xb * xb + 2 * aa * xb * pxb + ba * pxb * pxb);
+    const double jb = 0.5 * ((1 + ab * ab) / bb * yb * yb + 2 * ab * yb * pyb + bb * pyb * pyb);
+    f[28] = (float)sqrt(fmax(ja, 0.0));
+    f[29] = (float)sqrt(fmax(jb, 0.0));
+  }
+  __syncthreads();  // norm_s
+  if (i < n) {
+    if (raw) {
+#pragma unroll
+      for (int k = 0; k < BGT_MLP_FEATURES; k++) rs[tid * (BGT_MLP_FEATURES + 1) + k] = f[k];
+    }
+    if (x) {
+#pragma unroll
+      for (int c = 0; c < IN / 8; c++) {
+        uint4 pk;
+        bf16* h = reinterpret_cast<bf16*>(&pk);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const int k = 8 * c + j, kk = k < BGT_MLP_FEATURES ? k : 0;
+          h[j] = __float2bfloat16_rn(k < BGT_MLP_FEATURES ? (f[kk] - norm_s[0][kk]) * norm_s[1][kk] : 0.0f);
+        }
+        xs[tid * (IN / 8) + (c ^ (tid & 7))] = pk;
+      }
+    }
+  }
+  __syncthreads();
   if (x) {
-    uint4 pk[IN / 8];
-    bf16* h = reinterpret_cast<bf16*>(pk);
-    for (int k = 0; k < IN; k++)
-      h[k] = __float2bfloat16_rn(k < BGT_MLP_FEATURES ? ((float)f[k] - mean[k]) * inv_std[k] : 0.0f);
-    uint4* dst = reinterpret_cast<uint4*>(x + i * IN);
-    for (int q = 0; q < IN / 8; q++) dst[q] = pk[q];
+    uint4* dst = reinterpret_cast<uint4*>(x + i0 * IN);
+    for (int q = tid; q < rows * (IN / 8); q += FEAT_BLOCK) {
+      const int r = q / (IN / 8), c = q % (IN / 8);
+      dst[q] = xs[r * (IN / 8) + (c ^ (r & 7))];
+    }
+  }
+  if (raw) {
+    float* dst = raw + i0 * BGT_MLP_FEATURES;
+    for (int q = tid; q < rows * BGT_MLP_FEATURES; q += FEAT_BLOCK)
+      dst[q] = rs[(q / BGT_MLP_FEATURES) * (BGT_MLP_FEATURES + 1) + q % BGT_MLP_FEATURES];
   }
 }
 
@@ -1096,7 +1146,9 @@ int bgt_mlp_features(const double* d_vec0, const double* d_vec, int64_t n, int64
   if (!d_vec0 || !d_vec || !d_table || n < 0 || stride < n || n_variants <= 0) return BGT_EINVAL;
   if (d_x && (!d_mean || !d_inv_std || !aligned16(d_x))) return BGT_EINVAL;
   if (n == 0) return 0;
-  features_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+  const size_t smem = (d_x ? FEAT_BLOCK * IN * sizeof(bf16) : 0) +
+                      (d_raw ? FEAT_BLOCK * (BGT_MLP_FEATURES + 1) * sizeof(float) : 0);
+  features_kernel<<<(unsigned)((n + FEAT_BLOCK - 1) / FEAT_BLOCK), FEAT_BLOCK, smem, (cudaStream_t)stream>>>(
       d_vec0, d_vec, n, stride, d_variant, d_table, d_mean, d_inv_std, d_raw, reinterpret_cast<bf16*>(d_x));
   return cudaGetLastError() == cudaSuccess ? 0 : BGT_ECUDA;
 }
