@@ -50,6 +50,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -188,6 +189,17 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
                : "memory");
 }
+// 16 consecutive FP32 columns of this thread's tensor-memory lane
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
 // 32 consecutive FP32 columns of this thread's tensor-memory lane
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -232,6 +244,12 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&r)[64]) {
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+// The same with a 64-byte swizzle: rows of 64 bytes, atoms of 8 rows 512 B
+// apart, layout type 4.
+__device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
 }
 // Instruction descriptor, kind::f16: FP32 accumulator (bits 4-5 = 1), A and
 // B BF16 (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bit 17, M >> 4 at 24.
@@ -641,6 +659,350 @@ static cudaError_t launch_gemm(const bf16* A, int64_t lda, int64_t a_rows, const
   if (splits == 1 && kb_total <= GemmCfg<NT, true>::BRES_BLOCKS)
     return launch_gemm_kernel<NT, EPI, true>(ma, mb, mc, m_tiles, splits, kb_total, ep, err, st, wait_ns, skip_mma);
   return launch_gemm_kernel<NT, EPI, false>(ma, mb, mc, m_tiles, splits, kb_total, ep, err, st, wait_ns, skip_mma);
+}
+
+// ---------------------------------------------------------------------------
+// Inference: the three hidden layers and the output layer of 128 rows in one
+// CTA, no activation leaving the SM.
+//
+// As three GEMMs and a head kernel the activations made six trips through L2
+// and HBM (134 MB a layer at 262,144 rows), and each launch had its ramp and
+// tail.  Here a tile's activations stay in shared memory (a 128 x 256 bf16
+// buffer in the MMA's K-major 128-byte-swizzled layout: the input rows first,
+// then rewritten by each layer's epilogue) and only the weights stream, 288 KB
+// a tile from L2 through a ring of five 16 KB stages (a layer's outputs x 32
+// columns, 64-byte swizzle; all three layers do not fit beside the activations).
+//
+// One tile is a chain MMA -> epilogue -> MMA of ~13,000 cycles, 4,600 of them
+// MMA; so a CTA holds two tiles, each with its activation buffer and half of
+// tensor memory, and the MMA of one runs under the epilogue of the other.
+// FIGURES
+//
+// Roles (18 warps): 0 TMA producer, 1 MMA issuer, 2-9 hidden epilogues (two
+// per tensor-memory lane quarter, half of the columns each), 10-17 output
+// layer (half a row per thread; by four warps, a row per thread, it alone took
+// 109 us).  The sums are those of the separate kernels: K blocks in the same
+// order, the output layer's 32 partial sums of 8 columns in the order of
+// head_kernel's lanes and shuffles.
+constexpr int FWD_HIDDEN_WARPS = 8;
+constexpr int FWD_COLS = H / (FWD_HIDDEN_WARPS / 4);  // columns a hidden-epilogue warp handles
+constexpr int FWD_HEAD = 2 + FWD_HIDDEN_WARPS;         // first output-layer warp
+constexpr int FWD_THREADS = 32 * (FWD_HEAD + 8);
+constexpr int FWD_STAGES = 5;
+constexpr int FWD_WK = BK / 2;                 // columns of a weight stage
+constexpr uint32_t FWD_W_BYTES = H * FWD_WK * 2;
+constexpr uint32_t FWD_A_BLOCK = BM * BK * 2;  // 64 columns of a tile's activations
+constexpr uint32_t FWD_A_BYTES = 4 * FWD_A_BLOCK;
+constexpr int FWD_SMEM = FWD_STAGES * FWD_W_BYTES + 2 * FWD_A_BYTES + 1024;
+
+// two ReLU outputs as bf16, the first in the low half
+__device__ __forceinline__ uint32_t relu_bf16x2(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(fmaxf(a, 0.0f), fmaxf(b, 0.0f));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// bf16 (a ReLU output) rounded as the stored activation
+__device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+__global__ void __launch_bounds__(FWD_THREADS, 1)
+    forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW1,
+                   const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmW3, int n_tiles,
+                   const float* __restrict__ params, float* __restrict__ prob, int* err, uint64_t wait_ns) {
+  constexpr int S = FWD_STAGES;
+  constexpr uint32_t IDESC = idesc_bf16(BM, H);
+  extern __shared__ uint8_t smem_raw[];
+  // per slot p (tile in flight): x_full input rows landed, a_free its buffer
+  // may be loaded again, a_full block of activations written (two phases a
+  // tile), acc_full a layer's accumulators complete, acc_empty drained; per
+  // lane quarter, head_full / head_empty the hand-over of partial sums
+  __shared__ __align__(8) uint64_t w_full[S], w_empty[S], x_full[2], a_free[2], a_full[2], acc_full[2][3],
+      acc_empty[2], head_full[4], head_empty[4], done_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ __align__(16) float bias_s[3][H], w4_s[H];
+  __shared__ float head_s[8][BM];  // partial sums handed from one half of an output row to the other
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const uint32_t a_off = S * FWD_W_BYTES;  // slot p's activations at a_off + p * FWD_A_BYTES
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&tmem_slot), 2 * H);
+    tmem_relinquish();
+  }
+  // launched as a programmatic dependent, as gemm_kernel
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  for (int j = tid; j < H; j += FWD_THREADS) {
+    bias_s[0][j] = params[OFF_B1 + j];
+    bias_s[1][j] = params[OFF_B2 + j];
+    bias_s[2][j] = params[OFF_B3 + j];
+    w4_s[j] = round_bf16(params[OFF_W4 + j]);
+  }
+  if (tid == 0) {
+    for (int s = 0; s < S; s++) {
+      mbar_init(smem_u32(&w_full[s]), 1);
+      mbar_init(smem_u32(&w_empty[s]), 1);
+    }
+    for (int p = 0; p < 2; p++) {
+      mbar_init(smem_u32(&x_full[p]), 1);
+      mbar_init(smem_u32(&a_free[p]), 1);
+      mbar_init(smem_u32(&a_full[p]), FWD_HIDDEN_WARPS);
+      for (int k = 0; k < 3; k++) mbar_init(smem_u32(&acc_full[p][k]), 1);
+      mbar_init(smem_u32(&acc_empty[p]), FWD_HIDDEN_WARPS);
+    }
+    for (int k = 0; k < 4; k++) {
+      mbar_init(smem_u32(&head_full[k]), 1);
+      mbar_init(smem_u32(&head_empty[k]), 1);
+    }
+    mbar_init(smem_u32(&done_bar), 1);
+    fence_mbar_init();
+    prefetch_map(&tmX);
+    prefetch_map(&tmW1);
+    prefetch_map(&tmW2);
+    prefetch_map(&tmW3);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  bool ok = true;
+  // round i: slot 0 holds tile t0 + 2 i grid, slot 1 the one grid further (if any)
+  const int t0 = blockIdx.x, step = gridDim.x;
+
+  if (warp == 0) {
+    // ---------------- TMA producer ----------------
+    if (lane == 0) {
+      int it = 0;            // weight blocks issued
+      int nx[2] = {0, 0};    // input tiles issued
+      auto load_w = [&](const CUtensorMap* map, int kb) {
+        for (int k0 = kb * BK; k0 < (kb + 1) * BK; k0 += FWD_WK, it++) {
+          const int s = it % S;
+          if (!mbar_wait(smem_u32(&w_empty[s]), ((uint32_t)(it / S) & 1u) ^ 1u, wait_ns)) return false;
+          mbar_arrive_expect_tx(smem_u32(&w_full[s]), FWD_W_BYTES);
+          tma_load_2d(base + (uint32_t)s * FWD_W_BYTES, map, k0, 0, smem_u32(&w_full[s]));
+        }
+        return true;
+      };
+      // slot p's next input rows, once the last layer of its tile has read the buffer
+      auto load_x = [&](int p, int t) {
+        if (t >= n_tiles) return true;
+        if (!mbar_wait(smem_u32(&a_free[p]), ((uint32_t)nx[p] & 1u) ^ 1u, wait_ns)) return false;
+        mbar_arrive_expect_tx(smem_u32(&x_full[p]), FWD_A_BLOCK);
+        tma_load_2d(base + a_off + (uint32_t)p * FWD_A_BYTES, &tmX, 0, t * BM, smem_u32(&x_full[p]));
+        nx[p]++;
+        return true;
+      };
+      for (int t = t0; t < n_tiles && ok; t += 2 * step) {
+        const int slots = t + step < n_tiles ? 2 : 1;
+        // (the first weights are on their way before a buffer is waited for)
+        for (int p = 0; p < slots && ok; p++) ok = load_w(&tmW1, 0) && load_x(p, t + p * step);
+        for (int l = 0; l < 2 && ok; l++)
+          for (int p = 0; p < slots && ok; p++)
+            for (int kb = 0; kb < 4 && ok; kb++) ok = load_w(l == 0 ? &tmW2 : &tmW3, kb);
+      }
+      // every load issued has landed before the CTA can exit (bounded)
+      for (int s = 0; s < S && s < it; s++) {
+        const int last = it - 1 - ((it - 1 - s) % S);
+        mbar_wait(smem_u32(&w_full[s]), (uint32_t)(last / S) & 1u, wait_ns);
+      }
+      for (int p = 0; p < 2; p++)
+        if (nx[p] > 0) mbar_wait(smem_u32(&x_full[p]), (uint32_t)(nx[p] - 1) & 1u, wait_ns);
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    if (lane == 0) {
+      int it = 0, i = 0;  // weight blocks and rounds so far
+      bool issued = false;
+      for (int t = t0; t < n_tiles && ok; t += 2 * step, i++) {
+        const int slots = t + step < n_tiles ? 2 : 1;
+        for (int layer = 0; layer < 3 && ok; layer++) {
+          for (int p = 0; p < slots && ok; p++) {
+            // the slot's accumulators are drained (its use 3 i + layer)
+            if (!mbar_wait(smem_u32(&acc_empty[p]), ((uint32_t)(3 * i + layer) & 1u) ^ 1u, wait_ns)) ok = false;
+            const uint32_t d = tmem + (uint32_t)(p * H);
+            // its input rows or activations are in place
+            if (ok && !(layer == 0 ? mbar_wait(smem_u32(&x_full[p]), (uint32_t)i & 1u, wait_ns)
+                                   : mbar_wait(smem_u32(&a_full[p]), (uint32_t)(layer - 1) & 1u, wait_ns)))
+              ok = false;
+            for (int kb = 0; kb < (layer == 0 ? 1 : 4) && ok; kb++) {
+              const uint32_t sa = base + a_off + (uint32_t)p * FWD_A_BYTES + (uint32_t)kb * FWD_A_BLOCK;
+              for (int k0 = 0; k0 < BK && ok; k0 += FWD_WK, it++) {
+                const int s = it % S;
+                if (!mbar_wait(smem_u32(&w_full[s]), (uint32_t)(it / S) & 1u, wait_ns)) {
+                  ok = false;
+                  break;
+                }
+                tc_fence_after();
+                const uint32_t sb = base + (uint32_t)s * FWD_W_BYTES;
+#pragma unroll
+                for (int k = 0; k < FWD_WK / 16; k++)
+                  mma_bf16(d, sw128_desc(sa + 2 * k0 + k * 32), sw64_desc(sb + k * 32), IDESC,
+                           (kb > 0 || k0 > 0 || k > 0) ? 1u : 0u);
+                mma_commit(smem_u32(&w_empty[s]));
+                issued = true;
+              }
+            }
+            if (ok) mma_commit(smem_u32(&acc_full[p][layer]));
+            if (ok && layer == 2) mma_commit(smem_u32(&a_free[p]));
+          }
+        }
+      }
+      // every MMA issued has completed before tensor memory is freed (bounded)
+      if (issued) {
+        mma_commit(smem_u32(&done_bar));
+        mbar_wait(smem_u32(&done_bar), 0u, wait_ns);
+      }
+    }
+  } else {
+    const int q = warp & 3;  // tensor-memory lanes 32q .. 32q + 31 = tile rows
+    const int row = q * 32 + lane;
+    const bool head = warp >= FWD_HEAD;
+    const int col0 = head ? 0 : ((warp - 2) >> 2) * FWD_COLS;  // a hidden-epilogue warp's first column
+    int i = 0, n_head = 0;  // rounds, hand-overs
+    for (int t = t0; t < n_tiles && ok; t += 2 * step, i++) {
+      const int slots = t + step < n_tiles ? 2 : 1;
+      for (int layer = head ? 2 : 0; layer < (head ? 3 : 2) && ok; layer++) {
+        for (int p = 0; p < slots && ok; p++) {
+          if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_full[p][layer]), (uint32_t)i & 1u, wait_ns))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(p * H);
+          if (!head) {
+            // ---------------- hidden epilogue: bias, ReLU, bf16 into the activation buffer
+#pragma unroll 1
+            for (int c0 = col0; c0 < col0 + FWD_COLS; c0 += 32) {
+              uint32_t r[32];
+              tmem_ld32(taddr + c0, r);
+              uint8_t* dst = base_ptr + a_off + p * FWD_A_BYTES + (c0 / BK) * FWD_A_BLOCK + row * 128;
+              const int chunk = (c0 % BK) / 8;
+#pragma unroll
+              for (int c = 0; c < 4; c++) {
+                uint32_t pk[4];
+#pragma unroll
+                for (int j = 0; j < 8; j += 4) {
+                  const float4 bb = *reinterpret_cast<const float4*>(&bias_s[layer][c0 + 8 * c + j]);
+                  const uint32_t* v = &r[8 * c + j];
+                  pk[j / 2] = relu_bf16x2(__uint_as_float(v[0]) + bb.x, __uint_as_float(v[1]) + bb.y);
+                  pk[j / 2 + 1] = relu_bf16x2(__uint_as_float(v[2]) + bb.z, __uint_as_float(v[3]) + bb.w);
+                }
+                *reinterpret_cast<uint4*>(dst + (((chunk + c) ^ (row & 7)) << 4)) =
+                    make_uint4(pk[0], pk[1], pk[2], pk[3]);
+              }
+            }
+            // one fence for all of the warp's stores
+            fence_proxy_async();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(smem_u32(&acc_empty[p]));
+              mbar_arrive(smem_u32(&a_full[p]));
+            }
+          } else {
+            // ---------------- output layer: half of a row's partial sums
+            // (of 8 columns each), l = 8 hb + 0..7 and 16 more
+            const int hb = (warp - FWD_HEAD) >> 2;
+            float part[16];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              const int c0 = 64 * hb + 32 * (k & 1) + 128 * (k >> 1);
+              uint32_t r[32];
+              tmem_ld32(taddr + c0, r);
+#pragma unroll
+              for (int l = 0; l < 4; l++) {
+                float acc = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 8; j += 4) {
+                  const int c = c0 + 8 * l + j;
+                  const float4 bb = *reinterpret_cast<const float4*>(&bias_s[2][c]);
+                  const float4 w = *reinterpret_cast<const float4*>(&w4_s[c]);
+                  const uint32_t* v = &r[8 * l + j];
+                  const uint32_t a01 = relu_bf16x2(__uint_as_float(v[0]) + bb.x, __uint_as_float(v[1]) + bb.y);
+                  const uint32_t a23 = relu_bf16x2(__uint_as_float(v[2]) + bb.z, __uint_as_float(v[3]) + bb.w);
+                  acc += __uint_as_float(a01 << 16) * w.x;
+                  acc += __uint_as_float(a01 & 0xffff0000u) * w.y;
+                  acc += __uint_as_float(a23 << 16) * w.z;
+                  acc += __uint_as_float(a23 & 0xffff0000u) * w.w;
+                }
+                part[4 * k + l] = acc;
+              }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[p]));
+#pragma unroll
+            for (int l = 0; l < 8; l++) part[l] += part[l + 8];
+            const uint32_t hand = (uint32_t)n_head++ & 1u;
+            if (hb == 1) {
+              if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&head_empty[q]), hand ^ 1u, wait_ns))) {
+                ok = false;
+                break;
+              }
+#pragma unroll
+              for (int l = 0; l < 8; l++) head_s[l][row] = part[l];
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&head_full[q]));
+            } else {
+              if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&head_full[q]), hand, wait_ns))) {
+                ok = false;
+                break;
+              }
+#pragma unroll
+              for (int l = 0; l < 8; l++) part[l] += head_s[l][row];
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&head_empty[q]));
+#pragma unroll
+              for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+                for (int l = 0; l < o; l++) part[l] += part[l + o];
+              const float z = part[0] + params[OFF_B4];
+              prob[(int64_t)(t + p * step) * BM + row] = 1.0f / (1.0f + expf(-z));
+            }
+          }
+        }
+      }
+    }
+  }
+  if (!ok) atomicExch(err, 1);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem, 2 * H);
+  }
+}
+
+// p(lost) of n rows (n % 128 == 0) from X bf16 [n][64]
+static cudaError_t launch_forward(const bf16* X, int64_t n, const bf16* w1, const bf16* w2, const bf16* w3,
+                                  const float* params, float* prob, int* err, cudaStream_t st) {
+  CUtensorMap mx, m1, m2, m3;
+  auto weights = [](CUtensorMap* m, const bf16* w, uint64_t k) {
+    return make_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w, k, H, k, FWD_WK, H, CU_TENSOR_MAP_SWIZZLE_64B);
+  };
+  if (!(make_map(&mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, X, IN, (uint64_t)n, IN, BK, BM, CU_TENSOR_MAP_SWIZZLE_128B) &&
+        weights(&m1, w1, IN) && weights(&m2, w2, H) && weights(&m3, w3, H)))
+    return cudaErrorInvalidValue;
+  static std::atomic<bool> attr_set[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM);
+    if (e != cudaSuccess) return e;
+    attr_set[dev & 63].store(true, std::memory_order_release);
+  }
+  const int n_tiles = (int)(n / BM);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min(n_tiles, sm_count()));
+  cfg.blockDim = dim3(FWD_THREADS);
+  cfg.dynamicSmemBytes = FWD_SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, forward_kernel, mx, m1, m2, m3, n_tiles, params, prob, err, 2000000000ull);
 }
 
 // ---------------------------------------------------------------------------
@@ -1089,11 +1451,9 @@ int bgt_mlp_forward(bgt_mlp* m, const uint16_t* d_x, int64_t n, float* d_prob, v
   MCU(m, cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
   const bf16* X = reinterpret_cast<const bf16*>(d_x);
-  for (int64_t r0 = 0; r0 < n; r0 += m->max_batch) {
-    const int64_t rows = std::min<int64_t>(m->max_batch, n - r0);
-    int rc = forward_rows(m, X + r0 * IN, rows, false, nullptr, 0.0f, d_prob + r0, st);
-    if (rc) return rc;
-  }
+  if (n == 0) return 0;
+  MCU(m, launch_forward(X, n, m->w1, m->w2, m->w3, m->params, d_prob, m->d_err, st));
+  m->launches++;
   return 0;
 }
 

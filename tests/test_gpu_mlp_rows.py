@@ -42,3 +42,31 @@ def test_features_row_counts(n, raw, normalized):
         want = np.zeros((mlp.pad_rows(n), 64), np.float32)
         want[:n, :30] = (f32 - mean.astype(np.float32)) * (1.0 / std).astype(np.float32)
         assert torch.equal(x.cpu(), torch.tensor(want).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 147, 148, 149, 295, 296, 297, 593])
+def test_forward_does_not_depend_on_the_tile_schedule(tiles):
+    """Rows of a call over `tiles` 128-row tiles (one or two in flight per CTA,
+    an odd one left over, several rounds) equal the same rows alone."""
+    import torch
+
+    from bgt import mlp
+
+    net = mlp.SurvivalMLP(max_batch=128, seed=5)
+    g = torch.Generator().manual_seed(tiles)
+    x = torch.randn((128 * tiles, 64), generator=g).to(torch.bfloat16).cuda()
+    p = net.forward(x)
+    assert torch.isfinite(p).all() and 0 < p.min() and p.max() < 1
+    for t in sorted({0, 1, tiles // 3, tiles // 2, tiles - 2, tiles - 1} & set(range(tiles))):
+        assert torch.equal(p[128 * t:128 * (t + 1)], net.forward(x[128 * t:128 * (t + 1)].contiguous())), t
+    # against the layers in FP32 with activations rounded to bf16: rounding an activation to the other
+    # neighbour moves a logit by at most 2^-8 |a w|, and sums differ by reordering only
+    w = torch.from_numpy(net.get_params()).cuda()
+    a = x.float()
+    for o, cols in ((0, 64), (16640, 256), (82432, 256)):
+        W = w[o:o + 256 * cols].view(256, cols).to(torch.bfloat16).float()
+        a = torch.relu(a.double() @ W.double().T + w[o + 256 * cols:o + 256 * cols + 256].double()).to(
+            torch.bfloat16).float()
+    z = a @ w[148224:148480].to(torch.bfloat16).float() + w[148480]
+    bound = 2.0 ** -8 * (a.abs() @ w[148224:148480].abs()) * 0.25 * 4  # all four rounding points, slope 1/4
+    assert ((torch.sigmoid(z) - p).abs() <= bound + 1e-6).all()
