@@ -1008,105 +1008,217 @@ static cudaError_t launch_forward(const bf16* X, int64_t n, const bf16* w1, cons
 // ---------------------------------------------------------------------------
 // CUDA-core kernels
 
-// output layer, probability, loss and its gradient; one warp per sample
-__global__ void head_kernel(const bf16* __restrict__ A3, int64_t n, const float* __restrict__ w4,
-                            const float* __restrict__ b4, const float* __restrict__ label, float inv_batch,
-                            float* __restrict__ prob, float* __restrict__ dlogit, bf16* __restrict__ dz3,
-                            bf16* __restrict__ dz3_t, int64_t ldt, float* __restrict__ loss_acc) {
-  const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (s >= n) return;
-  const uint4 u = *reinterpret_cast<const uint4*>(A3 + s * H + lane * 8);
-  const bf16* a = reinterpret_cast<const bf16*>(&u);
-  float w[8], av[8];
-  float acc = 0.0f;
+// Output layer, loss and its gradient dZ3, row-major and transposed, of 64
+// samples per block (the first n / 64 blocks), and the transposed input Xt[k][s]
+// = X[s][k] of 64 samples (the next n / 64).  A warp takes eight samples; the
+// transposed copies pass through shared memory and leave in 16-byte stores, 64
+// samples of a column at a time (2-byte stores by the sample's own warp, and a
+// transpose launch of its own, took 39 us of a 8,192-sample step; 7 us now).
+constexpr int HEAD_ROWS = 64;
+__global__ void __launch_bounds__(256)
+    head_kernel(const bf16* __restrict__ A3, int64_t n, const float* __restrict__ w4, const float* __restrict__ b4,
+                const float* __restrict__ label, float inv_batch, float* __restrict__ dlogit, bf16* __restrict__ dz3,
+                bf16* __restrict__ dz3_t, const bf16* __restrict__ X, bf16* __restrict__ xt, int64_t ldt,
+                float* __restrict__ loss_acc) {
+  __shared__ __align__(16) bf16 tile[HEAD_ROWS][H];
+  __shared__ float loss_s[8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t n_head = n / HEAD_ROWS;
+  if (blockIdx.x >= n_head) {
+    bf16(*xs)[IN + 2] = reinterpret_cast<bf16(*)[IN + 2]>(tile);
+    const int64_t s0 = (blockIdx.x - n_head) * HEAD_ROWS;
+    for (int q = tid; q < HEAD_ROWS * IN / 8; q += 256) {
+      const uint4 u = reinterpret_cast<const uint4*>(X + s0 * IN)[q];
+      const bf16* h = reinterpret_cast<const bf16*>(&u);
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    w[j] = __bfloat162float(__float2bfloat16_rn(w4[lane * 8 + j]));
-    av[j] = __bfloat162float(a[j]);
-    acc += av[j] * w[j];
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  const float z = acc + b4[0];
-  const float p = 1.0f / (1.0f + expf(-z));
-  if (prob && lane == 0) prob[s] = p;
-  if (!label) return;
-  const float y = label[s];
-  const float g = (p - y) * inv_batch;
-  if (lane == 0) {
-    dlogit[s] = g;
-    // binary cross-entropy in the softplus form
-    const float l = fmaxf(z, 0.0f) - z * y + log1pf(expf(-fabsf(z)));
-    atomicAdd(loss_acc, l * inv_batch);
-  }
-  uint4 out;
-  bf16* o = reinterpret_cast<bf16*>(&out);
-#pragma unroll
-  for (int j = 0; j < 8; j++) o[j] = __float2bfloat16_rn(av[j] > 0.0f ? g * w[j] : 0.0f);
-  *reinterpret_cast<uint4*>(dz3 + s * H + lane * 8) = out;
-#pragma unroll
-  for (int j = 0; j < 8; j++) dz3_t[(int64_t)(lane * 8 + j) * ldt + s] = o[j];
-}
-
-// partial[c][j] = sum over rows s of chunk c of w[s] * M[s][j] (w = 1 if NULL)
-__global__ void colsum_kernel(const bf16* __restrict__ M, int64_t ldm, const float* __restrict__ w, int64_t n,
-                              int rows_per_chunk, int ncols, float* __restrict__ partial) {
-  const int j = threadIdx.x;
-  const int64_t c = blockIdx.x;
-  if (j >= ncols) return;
-  const int64_t s0 = c * rows_per_chunk, s1 = min(n, s0 + rows_per_chunk);
-  float acc = 0.0f;
-  for (int64_t s = s0; s < s1; s++) acc += (w ? w[s] : 1.0f) * __bfloat162float(M[s * ldm + j]);
-  partial[c * ncols + j] = acc;
-}
-
-// out[j] = sum_c partial[c][j], j < count
-__global__ void reduce_kernel(const float* __restrict__ partial, int64_t n_chunks, int64_t count,
-                              float* __restrict__ out) {
-  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j >= count) return;
-  float acc = 0.0f;
-  for (int64_t c = 0; c < n_chunks; c++) acc += partial[c * count + j];
-  out[j] = acc;
-}
-
-// sum of the first n floats into out[0] (one block)
-__global__ void sum_kernel(const float* __restrict__ x, int64_t n, float* __restrict__ out) {
-  __shared__ float sh[256];
-  float acc = 0.0f;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) acc += x[i];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+      for (int j = 0; j < 8; j++) xs[q / (IN / 8)][q % (IN / 8) * 8 + j] = h[j];
+    }
     __syncthreads();
+    const int k = tid >> 2, r0 = (tid & 3) * 16;
+#pragma unroll
+    for (int r = r0; r < r0 + 16; r += 8) {
+      uint4 u;
+      bf16* h = reinterpret_cast<bf16*>(&u);
+#pragma unroll
+      for (int j = 0; j < 8; j++) h[j] = xs[r + j][k];
+      *reinterpret_cast<uint4*>(xt + (int64_t)k * ldt + s0 + r) = u;
+    }
+    return;
   }
-  if (threadIdx.x == 0) out[0] = sh[0];
+  const int64_t s0 = blockIdx.x * (int64_t)HEAD_ROWS;
+  float w[8], loss = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; j++) w[j] = round_bf16(w4[lane * 8 + j]);
+  uint4 u[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) u[k] = *reinterpret_cast<const uint4*>(A3 + (s0 + warp * 8 + k) * H + lane * 8);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int r = warp * 8 + k;
+    const bf16* a = reinterpret_cast<const bf16*>(&u[k]);
+    float av[8], acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      av[j] = __bfloat162float(a[j]);
+      acc += av[j] * w[j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const float z = acc + b4[0];
+    const float p = 1.0f / (1.0f + expf(-z));
+    const float y = label[s0 + r];
+    const float g = (p - y) * inv_batch;
+    if (lane == 0) {
+      dlogit[s0 + r] = g;
+      // binary cross-entropy in the softplus form
+      loss += (fmaxf(z, 0.0f) - z * y + log1pf(expf(-fabsf(z)))) * inv_batch;
+    }
+    uint4 out;
+    bf16* o = reinterpret_cast<bf16*>(&out);
+#pragma unroll
+    for (int j = 0; j < 8; j++) o[j] = __float2bfloat16_rn(av[j] > 0.0f ? g * w[j] : 0.0f);
+    *reinterpret_cast<uint4*>(dz3 + (s0 + r) * H + lane * 8) = out;
+    *reinterpret_cast<uint4*>(&tile[r][lane * 8]) = out;
+  }
+  if (lane == 0) loss_s[warp] = loss;
+  __syncthreads();
+  if (tid == 0) {
+    for (int k = 1; k < 8; k++) loss += loss_s[k];
+    atomicAdd(loss_acc, loss);
+  }
+  bf16* dst = dz3_t + (int64_t)tid * ldt + s0;
+#pragma unroll
+  for (int r = 0; r < HEAD_ROWS; r += 8) {
+    uint4 v;
+    bf16* h = reinterpret_cast<bf16*>(&v);
+#pragma unroll
+    for (int j = 0; j < 8; j++) h[j] = tile[r + j][tid];
+    *reinterpret_cast<uint4*>(dst + r) = v;
+  }
 }
 
-// Xt[k][s] = X[s][k]
-__global__ void transpose_in_kernel(const bf16* __restrict__ X, int64_t n, bf16* __restrict__ Xt, int64_t ldt) {
-  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  for (int k = 0; k < IN; k++) Xt[(int64_t)k * ldt + s] = X[s * IN + k];
+// Column sums over 128 rows (blockIdx.x) of dZ1, dZ2, dZ3 and of A3 weighted by
+// dlogit (blockIdx.y): partial[y][x][j], rows added in order.  16 rows' loads
+// are in flight at a time (one at a time, in four launches: 78 us of a
+// 8,192-sample step).
+__global__ void __launch_bounds__(H / 2)
+    colsum_kernel(const bf16* __restrict__ dz1, const bf16* __restrict__ dz2, const bf16* __restrict__ dz3,
+                  const bf16* __restrict__ a3, const float* __restrict__ dlogit, float* __restrict__ partial) {
+  const int y = blockIdx.y, j = threadIdx.x;
+  const int64_t s0 = blockIdx.x * (int64_t)128;
+  const bf16* M = (y == 0 ? dz1 : y == 1 ? dz2 : y == 2 ? dz3 : a3) + s0 * H + 2 * j;
+  float acc0 = 0.0f, acc1 = 0.0f;
+  for (int s = 0; s < 128; s += 16) {
+    __nv_bfloat162 v[16];
+    float w[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      v[k] = *reinterpret_cast<const __nv_bfloat162*>(M + (int64_t)(s + k) * H);
+      w[k] = y == 3 ? dlogit[s0 + s + k] : 1.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      acc0 += w[k] * __bfloat162float(v[k].x);
+      acc1 += w[k] * __bfloat162float(v[k].y);
+    }
+  }
+  float* out = partial + ((int64_t)y * gridDim.x + blockIdx.x) * H + 2 * j;
+  out[0] = acc0;
+  out[1] = acc1;
 }
 
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, int64_t n, float lr, float b1, float b2, float eps, float bc1,
-                            float bc2) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-}
+// Adam's constants of a step; lr = 0 with train = 0: gradients only
+struct AdamStep {
+  int train;
+  float lr, bc1, bc2;
+};
 
-// bf16 weights for the GEMMs: W (row-major [out][in]) and, for the hidden
-// layers, W^T ([in][out]) for the backward pass
+// The gradients from their partial sums, and with train the Adam update and
+// the bf16 weights (W row-major [out][in] and, for the hidden layers, W^T) for
+// the next step: one pass over the parameters, one block per 256 of them
+// (every parameter array starts on a multiple of 256), and a last block for
+// b4 = sum dlogit.  As seven reductions, Adam and packing they were launches
+// that each waited for the one before: 66 us of a 8,192-sample step.
+// Partial sums are added in order, so the gradients are deterministic.
+__global__ void __launch_bounds__(256)
+    finish_kernel(const float* __restrict__ p1, const float* __restrict__ p2, const float* __restrict__ p3, int splits,
+                  const float* __restrict__ pc, int chunks, const float* __restrict__ dlogit, int64_t batch,
+                  float* __restrict__ grads, float* __restrict__ params, float* __restrict__ adam_m,
+                  float* __restrict__ adam_v, bf16* __restrict__ w1, bf16* __restrict__ w2, bf16* __restrict__ w2t,
+                  bf16* __restrict__ w3, bf16* __restrict__ w3t, AdamStep step) {
+  __shared__ float sh[256];
+  const int64_t i0 = blockIdx.x * (int64_t)256;
+  const int tid = threadIdx.x;
+  int64_t i = i0 + tid;
+  float g = 0.0f;
+  if (i0 == OFF_B4) {
+    for (int64_t k = tid; k < batch; k += 256) g += dlogit[k];
+    sh[tid] = g;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if (tid < o) sh[tid] += sh[tid + o];
+      __syncthreads();
+    }
+    if (tid != 0) return;
+    g = sh[0];
+  } else {
+    const float* src;
+    int64_t stride;
+    int count;
+    const auto weights = [&](const float* p, int64_t off, int64_t size) {
+      src = p + (i - off);
+      stride = size;
+      count = splits;
+    };
+    const auto columns = [&](int y, int64_t off) {
+      src = pc + (int64_t)y * chunks * H + (i - off);
+      stride = H;
+      count = chunks;
+    };
+    if (i0 < OFF_B1) weights(p1, OFF_W1, (int64_t)H * IN);
+    else if (i0 < OFF_W2) columns(0, OFF_B1);
+    else if (i0 < OFF_B2) weights(p2, OFF_W2, (int64_t)H * H);
+    else if (i0 < OFF_W3) columns(1, OFF_B2);
+    else if (i0 < OFF_B3) weights(p3, OFF_W3, (int64_t)H * H);
+    else if (i0 < OFF_W4) columns(2, OFF_B3);
+    else columns(3, OFF_W4);
+    int c = 0;
+    for (; c + 16 <= count; c += 16) {
+      float v[16];
+#pragma unroll
+      for (int k = 0; k < 16; k++) v[k] = src[(c + k) * stride];
+#pragma unroll
+      for (int k = 0; k < 16; k++) g += v[k];
+    }
+    for (; c < count; c++) g += src[c * stride];
+  }
+  grads[i] = g;
+  if (!step.train) return;
+  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  const float mi = b1 * adam_m[i] + (1.0f - b1) * g;
+  const float vi = b2 * adam_v[i] + (1.0f - b2) * g * g;
+  adam_m[i] = mi;
+  adam_v[i] = vi;
+  const float pi = params[i] - step.lr * (mi / step.bc1) / (sqrtf(vi / step.bc2) + eps);
+  params[i] = pi;
+  const bf16 h = __float2bfloat16_rn(pi);
+  if (i0 < OFF_B1) {
+    w1[i] = h;
+  } else if (i0 >= OFF_W2 && i0 < OFF_B2) {
+    i -= OFF_W2;
+    w2[i] = h;
+    w2t[(i % H) * H + i / H] = h;
+  } else if (i0 >= OFF_W3 && i0 < OFF_B3) {
+    i -= OFF_W3;
+    w3[i] = h;
+    w3t[(i % H) * H + i / H] = h;
+  }
+}
+static_assert(OFF_B1 % 256 == 0 && OFF_W2 % 256 == 0 && OFF_B2 % 256 == 0 && OFF_W3 % 256 == 0 && OFF_B3 % 256 == 0 &&
+                  OFF_W4 % 256 == 0 && OFF_B4 % 256 == 0,
+              "a block of finish_kernel lies in one parameter array");
+
+// bf16 weights for the GEMMs from the master parameters
 __global__ void pack_kernel(const float* __restrict__ p, bf16* __restrict__ w1, bf16* __restrict__ w2,
                             bf16* __restrict__ w2t, bf16* __restrict__ w3, bf16* __restrict__ w3t) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1246,6 +1358,12 @@ static cudaError_t mlp_alloc(bgt_mlp* m, T** p, size_t count) {
   return e;
 }
 
+// splits of a weight gradient over a batch: one chunk per CTA of a full wave,
+// at least KSPLIT samples each
+static int64_t max_splits(int64_t batch) {
+  return std::max<int64_t>(1, std::min<int64_t>(batch / KSPLIT, sm_count() / (H / BM)));
+}
+
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 // splitmix64 -> uniform in [-1, 1)
@@ -1274,8 +1392,8 @@ int bgt_mlp_create(bgt_mlp** out, int32_t max_batch, uint64_t seed, int32_t devi
   m->max_batch = max_batch;
   cudaError_t e = cudaSetDevice(device);
   const int64_t B = max_batch;
-  const int64_t n_split = B / KSPLIT;
-  const int64_t partial = std::max<int64_t>(n_split * 2 * BM * H, (B / 128 + 1) * H);
+  // partial sums of a step: the three weight gradients' splits, four column sums
+  const int64_t partial = max_splits(B) * ((int64_t)H * IN + 2 * (int64_t)H * H) + (B / 128) * 4 * H;
   if (e == cudaSuccess) e = mlp_alloc(m, &m->params, N_PARAMS);
   if (e == cudaSuccess) e = mlp_alloc(m, &m->grads, N_PARAMS);
   if (e == cudaSuccess) e = mlp_alloc(m, &m->adam_m, N_PARAMS);
@@ -1344,32 +1462,6 @@ int bgt_mlp_set_params(bgt_mlp* m, const float* params) {
 
 }  // extern "C"
 
-// forward pass of n rows (n % 128 == 0, n <= max_batch when training) from
-// X bf16 [n][64]; training keeps the transposed copies for the weight
-// gradients and runs the loss head with labels
-static int forward_rows(bgt_mlp* m, const bf16* X, int64_t n, bool training, const float* label, float inv_batch,
-                        float* prob, cudaStream_t st) {
-  const int64_t ldt = m->max_batch;
-  Epi e{};
-  e.bias = m->params + OFF_B1;
-  e.out_t = training ? m->a1t : nullptr;
-  e.ldt = ldt;
-  MCU(m, (launch_gemm<256, EPI_FWD>(X, IN, n, m->w1, IN, IN, 1, m->a1, H, e, m->d_err, st)));
-  e.bias = m->params + OFF_B2;
-  e.out_t = training ? m->a2t : nullptr;
-  MCU(m, (launch_gemm<256, EPI_FWD>(m->a1, H, n, m->w2, H, H, 1, m->a2, H, e, m->d_err, st)));
-  e.bias = m->params + OFF_B3;
-  e.out_t = nullptr;
-  MCU(m, (launch_gemm<256, EPI_FWD>(m->a2, H, n, m->w3, H, H, 1, m->a3, H, e, m->d_err, st)));
-  const int64_t threads = n * 32;
-  head_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(
-      m->a3, n, m->params + OFF_W4, m->params + OFF_B4, label, inv_batch, prob, m->dlogit, m->dz3, m->dz3t, ldt,
-      m->scalars);
-  m->launches += 4;
-  MCU(m, cudaGetLastError());
-  return 0;
-}
-
 static int check_error_flag(bgt_mlp* m) {
   int flag = 0;
   MCU(m, cudaMemcpy(&flag, m->d_err, sizeof(int), cudaMemcpyDeviceToHost));
@@ -1377,16 +1469,30 @@ static int check_error_flag(bgt_mlp* m) {
   return 0;
 }
 
-// gradients of the mean loss over one batch into m->grads
-static int backward_batch(bgt_mlp* m, const bf16* X, const float* label, int32_t batch, cudaStream_t st) {
+// Gradients of the mean loss over one batch into `grads`; with step.train the
+// Adam update and the packed weights as well.
+static int train_batch(bgt_mlp* m, const bf16* X, const float* label, int32_t batch, float* grads, AdamStep step,
+                       cudaStream_t st) {
   const int64_t B = batch, ldt = m->max_batch;
   MCU(m, cudaMemsetAsync(m->scalars, 0, sizeof(float), st));
-  transpose_in_kernel<<<(unsigned)((B + 255) / 256), 256, 0, st>>>(X, B, m->xt, ldt);
-  m->launches++;
-  int rc = forward_rows(m, X, B, true, label, 1.0f / (float)B, nullptr, st);
-  if (rc) return rc;
-  // dZ2 = (dZ3 . W3) * relu'(A2), dZ1 = (dZ2 . W2) * relu'(A1)
+  // forward, with transposed copies of the activations for the weight gradients
   Epi e{};
+  e.bias = m->params + OFF_B1;
+  e.out_t = m->a1t;
+  e.ldt = ldt;
+  MCU(m, (launch_gemm<256, EPI_FWD>(X, IN, B, m->w1, IN, IN, 1, m->a1, H, e, m->d_err, st)));
+  e.bias = m->params + OFF_B2;
+  e.out_t = m->a2t;
+  MCU(m, (launch_gemm<256, EPI_FWD>(m->a1, H, B, m->w2, H, H, 1, m->a2, H, e, m->d_err, st)));
+  e.bias = m->params + OFF_B3;
+  e.out_t = nullptr;
+  MCU(m, (launch_gemm<256, EPI_FWD>(m->a2, H, B, m->w3, H, H, 1, m->a3, H, e, m->d_err, st)));
+  head_kernel<<<(unsigned)(2 * (B / HEAD_ROWS)), 256, 0, st>>>(
+      m->a3, B, m->params + OFF_W4, m->params + OFF_B4, label, 1.0f / (float)B, m->dlogit, m->dz3, m->dz3t, X, m->xt,
+      ldt, m->scalars);
+  MCU(m, cudaGetLastError());
+  // dZ2 = (dZ3 . W3) * relu'(A2), dZ1 = (dZ2 . W2) * relu'(A1)
+  e = Epi{};
   e.ldt = ldt;
   e.ldm = H;
   e.out_t = m->dz2t;
@@ -1395,41 +1501,23 @@ static int backward_batch(bgt_mlp* m, const bf16* X, const float* label, int32_t
   e.out_t = m->dz1t;
   e.mask = m->a1;
   MCU(m, (launch_gemm<256, EPI_BWD>(m->dz2, H, B, m->w2t, H, H, 1, m->dz1, H, e, m->d_err, st)));
-  // weight gradients dW = dZ^T . A_prev over the batch, split into one
-  // chunk per CTA of a full wave (at least KSPLIT samples per chunk: the
-  // partial buffer holds max_batch / KSPLIT chunks); the FP32 partials are
-  // summed in a fixed order, so the gradients are deterministic
-  const int splits = (int)std::max<int64_t>(1, std::min<int64_t>(B / KSPLIT, sm_count() / (H / BM)));
-  Epi f{};
-  struct G {
-    const bf16* dzt;
-    const bf16* at;
-    int64_t off;
-    int nt;
-  } gs[3] = {{m->dz3t, m->a2t, OFF_W3, 256}, {m->dz2t, m->a1t, OFF_W2, 256}, {m->dz1t, m->xt, OFF_W1, 64}};
-  for (const G& g : gs) {
-    if (g.nt == 256)
-      MCU(m, (launch_gemm<256, EPI_F32>(g.dzt, ldt, H, g.at, ldt, B, splits, m->partial, 256, f, m->d_err, st)));
-    else
-      MCU(m, (launch_gemm<64, EPI_F32>(g.dzt, ldt, H, g.at, ldt, B, splits, m->partial, 64, f, m->d_err, st)));
-    const int64_t count = (int64_t)H * g.nt;
-    reduce_kernel<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(m->partial, splits, count, m->grads + g.off);
-    m->launches += 2;
-  }
-  // bias gradients (column sums of dZ), output layer w4 = sum dlogit * A3, b4 = sum dlogit
+  // weight gradients dW = dZ^T . A_prev over the batch as FP32 partial sums
+  const int splits = (int)max_splits(B);
   const int chunks = (int)(B / 128);
-  struct C2 {
-    const bf16* mat;
-    const float* w;
-    int64_t off;
-  } cs[4] = {{m->dz1, nullptr, OFF_B1}, {m->dz2, nullptr, OFF_B2}, {m->dz3, nullptr, OFF_B3}, {m->a3, m->dlogit, OFF_W4}};
-  for (const C2& c : cs) {
-    colsum_kernel<<<chunks, 256, 0, st>>>(c.mat, H, c.w, B, 128, H, m->partial);
-    reduce_kernel<<<1, 256, 0, st>>>(m->partial, chunks, H, m->grads + c.off);
-    m->launches += 2;
-  }
-  sum_kernel<<<1, 256, 0, st>>>(m->dlogit, B, m->grads + OFF_B4);
-  m->launches++;
+  float* p3 = m->partial;
+  float* p2 = p3 + (int64_t)splits * H * H;
+  float* p1 = p2 + (int64_t)splits * H * H;
+  float* pc = p1 + (int64_t)splits * H * IN;
+  const Epi f{};
+  MCU(m, (launch_gemm<256, EPI_F32>(m->dz3t, ldt, H, m->a2t, ldt, B, splits, p3, 256, f, m->d_err, st)));
+  MCU(m, (launch_gemm<256, EPI_F32>(m->dz2t, ldt, H, m->a1t, ldt, B, splits, p2, 256, f, m->d_err, st)));
+  MCU(m, (launch_gemm<64, EPI_F32>(m->dz1t, ldt, H, m->xt, ldt, B, splits, p1, 64, f, m->d_err, st)));
+  // bias gradients (column sums of dZ), w4's = sum dlogit * A3
+  colsum_kernel<<<dim3((unsigned)chunks, 4), H / 2, 0, st>>>(m->dz1, m->dz2, m->dz3, m->a3, m->dlogit, pc);
+  finish_kernel<<<(unsigned)(OFF_B4 / 256 + 1), 256, 0, st>>>(p1, p2, p3, splits, pc, chunks, m->dlogit, B, grads,
+                                                             m->params, m->adam_m, m->adam_v, m->w1, m->w2, m->w2t,
+                                                             m->w3, m->w3t, step);
+  m->launches += 11;
   MCU(m, cudaGetLastError());
   return 0;
 }
@@ -1463,9 +1551,8 @@ int bgt_mlp_gradients(bgt_mlp* m, const uint16_t* d_x, const float* d_label, int
   if (rc) return rc;
   MCU(m, cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
-  rc = backward_batch(m, reinterpret_cast<const bf16*>(d_x), d_label, batch, st);
+  rc = train_batch(m, reinterpret_cast<const bf16*>(d_x), d_label, batch, d_grad ? d_grad : m->grads, AdamStep{}, st);
   if (rc) return rc;
-  if (d_grad) MCU(m, cudaMemcpyAsync(d_grad, m->grads, N_PARAMS * sizeof(float), cudaMemcpyDeviceToDevice, st));
   if (loss) {
     MCU(m, cudaMemcpyAsync(loss, m->scalars, sizeof(float), cudaMemcpyDeviceToHost, st));
     MCU(m, cudaStreamSynchronize(st));
@@ -1480,18 +1567,15 @@ int bgt_mlp_train_step(bgt_mlp* m, const uint16_t* d_x, const float* d_label, in
   if (rc) return rc;
   MCU(m, cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
-  rc = backward_batch(m, reinterpret_cast<const bf16*>(d_x), d_label, batch, st);
-  if (rc) return rc;
   m->step++;
   const float b1 = 0.9f, b2 = 0.999f;
   const float bc1 = 1.0f - (float)std::pow((double)b1, (double)m->step);
   const float bc2 = 1.0f - (float)std::pow((double)b2, (double)m->step);
-  adam_kernel<<<(unsigned)((N_PARAMS + 255) / 256), 256, 0, st>>>(m->params, m->grads, m->adam_m, m->adam_v,
-                                                                    N_PARAMS, lr, b1, b2, 1e-8f, bc1, bc2);
-  m->launches++;
-  MCU(m, cudaGetLastError());
-  rc = pack_weights(m, st);
-  if (rc) return rc;
+  rc = train_batch(m, reinterpret_cast<const bf16*>(d_x), d_label, batch, m->grads, AdamStep{1, lr, bc1, bc2}, st);
+  if (rc) {
+    m->step--;
+    return rc;
+  }
   if (loss) {
     MCU(m, cudaMemcpyAsync(loss, m->scalars, sizeof(float), cudaMemcpyDeviceToHost, st));
     MCU(m, cudaStreamSynchronize(st));
