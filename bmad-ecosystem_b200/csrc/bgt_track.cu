@@ -37,13 +37,10 @@ struct CallCtx {
   cudaEvent_t done = nullptr;
   bool used = false;             // `done` has been recorded
   int32_t* d_scratch = nullptr;  // [0] tile counter, [1] error flag, [2] status read-back
-  // device staging of host-buffer calls
-  double* d_vec6 = nullptr;
-  double* d_beta = nullptr;
-  int32_t* d_i32 = nullptr;  // state, ixe, ixt, slot map, tile variant
-  uint64_t* d_t = nullptr;   // particle times (binary128), cap of them
-  int64_t cap = 0, cap_slots = 0, cap_tiles = 0;
-  // pinned host staging of host-buffer calls
+  // device staging of host-buffer calls and scans (StageLayout)
+  unsigned char* d_stage = nullptr;
+  size_t stage_bytes = 0;
+  // pinned host staging of host-buffer calls, the same layout
   unsigned char* h_pin = nullptr;
   size_t pin_bytes = 0;
   // device-buffer calls: grouping by variant (slot map, tile variant; per
@@ -108,10 +105,7 @@ static void free_ctx(CallCtx* c) {
   if (c->st) cudaStreamDestroy(c->st);
   if (c->done) cudaEventDestroy(c->done);
   cudaFree(c->d_scratch);
-  cudaFree(c->d_vec6);
-  cudaFree(c->d_beta);
-  cudaFree(c->d_i32);
-  cudaFree(c->d_t);
+  cudaFree(c->d_stage);
   cudaFree(c->d_grp);
   cudaFree(c->d_grp_v);
   if (c->h_pin) cudaFreeHost(c->h_pin);
@@ -300,10 +294,10 @@ static int pick_kernel(bgt_handle* h, const bgt_tuning& tun, bool compact, bool 
   return 0;
 }
 
-// Enqueue tracking of slots on `st` with the call context's tile counter
-// and error flag.
-static int enqueue_track(bgt_handle* h, const bgt_tuning& tun, CallCtx* c, KArgs a, int64_t n_tiles,
-                         cudaStream_t st) {
+// Enqueue tracking of slots on `st` with the call's scratch words: [0] tile
+// counter (cleared here unless it is known to be zero), [1] error flag.
+static int enqueue_track(bgt_handle* h, const bgt_tuning& tun, int32_t* scratch, bool zeroed, KArgs a,
+                         int64_t n_tiles, cudaStream_t st) {
   LaunchFn launch = nullptr;
   size_t smem = 0;
   // the RARE instances also carry the particle time
@@ -313,11 +307,11 @@ static int enqueue_track(bgt_handle* h, const bgt_tuning& tun, CallCtx* c, KArgs
   int64_t grid = (int64_t)h->num_sms * std::max(1, tun.blocks_per_sm);
   if (grid > n_tiles) grid = n_tiles;
   if (grid < 1) grid = 1;
-  a.tile_counter = c->d_scratch;
-  a.error_flag = c->d_scratch + 1;
+  a.tile_counter = scratch;
+  a.error_flag = scratch + 1;
   a.wait_ns = wait_ns_of(tun);
   a.skip_table_copy = tun.test_skip_table_copy;
-  CU(h, cudaMemsetAsync(c->d_scratch, 0, sizeof(int32_t), st));
+  if (!zeroed) CU(h, cudaMemsetAsync(scratch, 0, sizeof(int32_t), st));
   const cudaError_t e = launch(a, (int)grid, smem, st);
   if (e != cudaSuccess) return set_err(h, BGT_ECUDA, std::string("track_kernel launch: ") + cudaGetErrorString(e));
   h->launches++;
@@ -360,6 +354,39 @@ static int normalise_tuning(bgt_handle* h, bgt_tuning* n) {
   if (n->test_skip_table_copy != 0 && n->test_skip_table_copy != 1)
     return set_err(h, BGT_EINVAL, "test_skip_table_copy must be 0 or 1");
   return 0;
+}
+
+// The particles of a host-buffer call or a scan, one block of memory: times
+// [n][16 B] (when tracked), vec6 [6][n], beta [n], state / ix_ele_lost /
+// ix_turn_lost [n] each, the kernel's scratch words, then the slot map and the
+// tile variants.  The same layout in pinned host memory and on the device, so
+// a call is one copy in (the scratch words arrive as zeros) and one copy back
+// (without the maps, the error flag among them): with a copy per array and two
+// memsets a call over 101 particles took 67 us, now 42.
+struct StageLayout {
+  size_t t, vec6, beta, state, ixe, ixt, scratch, slot, tvar, bytes;
+  StageLayout(int64_t n, int64_t n_slots, int64_t n_tiles, bool with_t) {
+    size_t o = 0;
+    auto place = [&](size_t bytes) {
+      const size_t at = o;
+      o += bytes;
+      return at;
+    };
+    t = place(with_t ? (size_t)n * 16 : 0);
+    vec6 = place((size_t)n * 48);
+    beta = place((size_t)n * 8);
+    state = place((size_t)n * 4);
+    ixe = place((size_t)n * 4);
+    ixt = place((size_t)n * 4);
+    scratch = place(16);
+    slot = place((size_t)n_slots * 4);
+    tvar = place((size_t)n_tiles * 4);
+    bytes = o;
+  }
+};
+template <class T>
+static T* at(unsigned char* base, size_t offset) {
+  return reinterpret_cast<T*>(base + offset);
 }
 
 extern "C" {
@@ -456,8 +483,10 @@ int64_t bgt_kernel_launch_count(const bgt_handle* h) { return h ? h->launches.lo
 
 // Track device-resident particles for turns [turn0, turn0 + n_turns) in
 // segments of tuning.turns_per_launch turns (one persistent launch each).
-// The call's error flag is cleared once, the tile counter per launch.
-static int track_device_impl(bgt_handle* h, const bgt_tuning& tun, CallCtx* c, int32_t* status, double* d_vec6,
+// The call's scratch words are zero (zeroed) or cleared here: the error flag
+// once, the tile counter per launch.
+static int track_device_impl(bgt_handle* h, const bgt_tuning& tun, int32_t* scratch, bool zeroed, int32_t* status,
+                             double* d_vec6,
                              int64_t n_stride, double* d_beta, uint64_t* d_t, int32_t* d_state, int32_t* d_ixe,
                              int32_t* d_ixt,
                              const int32_t* d_slot, const int32_t* d_tile_var, int64_t n, int64_t n_slots,
@@ -478,13 +507,13 @@ static int track_device_impl(bgt_handle* h, const bgt_tuning& tun, CallCtx* c, i
   a.rec_begin = rec_begin;
   a.rec_end = rec_end;
   a.status = status;
-  CU(h, cudaMemsetAsync(c->d_scratch + 1, 0, sizeof(int32_t), st));
+  if (!zeroed) CU(h, cudaMemsetAsync(scratch, 0, 2 * sizeof(int32_t), st));
   int64_t n_tiles = (n_slots + tun.threads_per_block - 1) / tun.threads_per_block;
   int32_t seg = tun.turns_per_launch > 0 ? tun.turns_per_launch : n_turns;
   for (int32_t t = 0; t < n_turns; t += seg) {
     a.turn0 = turn0 + t;
     a.n_turns = std::min(seg, n_turns - t);
-    int rc = enqueue_track(h, tun, c, a, n_tiles, st);
+    int rc = enqueue_track(h, tun, scratch, t == 0, a, n_tiles, st);
     if (rc) return rc;
   }
   return 0;
@@ -536,7 +565,7 @@ int bgt_track_turns_device(bgt_handle* h, double* d_vec6, double* d_beta, void* 
   CU(h, L.use(st));
   if (!d_variant || h->n_variants == 1) {
     tun = call_tuning(h, tun, {n}, tq != nullptr);
-    return track_device_impl(h, tun, c, h->d_status, d_vec6, n, d_beta, tq, d_state, d_ix_ele_lost,
+    return track_device_impl(h, tun, c->d_scratch, false, h->d_status, d_vec6, n, d_beta, tq, d_state, d_ix_ele_lost,
                              d_ix_turn_lost, nullptr, nullptr, n, n, turn0, n_turns, 0, h->n_ele, st);
   }
   // Group by variant into tile-aligned slot ranges.  The variant ids must be
@@ -586,7 +615,7 @@ int bgt_track_turns_device(bgt_handle* h, double* d_vec6, double* d_beta, void* 
   h->launches++;
   // (copies from pageable host memory return once the data is staged, so
   // slot0 and tvar may go out of scope before the copies complete)
-  return track_device_impl(h, tun, c, h->d_status, d_vec6, n, d_beta, tq, d_state, d_ix_ele_lost, d_ix_turn_lost,
+  return track_device_impl(h, tun, c->d_scratch, false, h->d_status, d_vec6, n, d_beta, tq, d_state, d_ix_ele_lost, d_ix_turn_lost,
                            d_slot, d_tvar, n, n_slots, turn0, n_turns, 0, h->n_ele, st);
 }
 
@@ -611,25 +640,15 @@ int bgt_device_status(bgt_handle* h, void* stream) {
   return 0;
 }
 
-// Grow a context's device staging buffers.
-static int ensure_staging(bgt_handle* h, CallCtx* c, int64_t n, int64_t n_slots, int64_t n_tiles, bool with_t) {
-  if (n <= c->cap && n_slots <= c->cap_slots && n_tiles <= c->cap_tiles && (!with_t || c->d_t)) return 0;
+// Grow a context's device staging block.
+static int ensure_staging(bgt_handle* h, CallCtx* c, size_t bytes) {
+  if (bytes <= c->stage_bytes) return 0;
   CU(h, cudaStreamSynchronize(c->st));
-  cudaFree(c->d_vec6);
-  cudaFree(c->d_beta);
-  cudaFree(c->d_i32);
-  cudaFree(c->d_t);
-  c->d_vec6 = nullptr;
-  c->d_beta = nullptr;
-  c->d_i32 = nullptr;
-  c->d_t = nullptr;
-  c->cap = std::max(n, c->cap);
-  c->cap_slots = std::max(n_slots, c->cap_slots);
-  c->cap_tiles = std::max(n_tiles, c->cap_tiles);
-  CU(h, cudaMalloc(&c->d_vec6, (size_t)c->cap * 6 * 8));
-  CU(h, cudaMalloc(&c->d_beta, (size_t)c->cap * 8));
-  CU(h, cudaMalloc(&c->d_i32, (size_t)(3 * c->cap + c->cap_slots + c->cap_tiles) * 4));
-  if (with_t) CU(h, cudaMalloc(&c->d_t, (size_t)c->cap * 16));
+  cudaFree(c->d_stage);
+  c->d_stage = nullptr;
+  c->stage_bytes = 0;
+  CU(h, cudaMalloc(&c->d_stage, bytes));
+  c->stage_bytes = bytes;
   return 0;
 }
 
@@ -725,77 +744,44 @@ static int track_host(bgt_handle* h, double* vec6, double* beta, void* t, int32_
       if (variant[i] != 0) return set_err(h, BGT_EINVAL, "variant out of range");
   }
   if (!multi) tun = call_tuning(h, tun, {n}, t != nullptr);
-  const int block = tun.threads_per_block;
-  int64_t n_tiles = (n_slots + block - 1) / block;
   CtxLease L(h);
   int rc = L.acquire();
   if (rc) return rc;
   CallCtx* c = L.c;
   cudaStream_t st = c->st;
   CU(h, L.use(st));
-  if ((rc = ensure_staging(h, c, n, n_slots, n_tiles, t != nullptr))) return rc;
-  // pinned layout: times [n][16 B] (when tracked), vec6 [6][n], beta [n],
-  // state/ixe/ixt [n] each, slot map, tile variants, error flag
-  const size_t b_t = t ? (size_t)n * 16 : 0;
-  const size_t b_v = (size_t)n * 6 * 8, b_b = (size_t)n * 8, b_i = (size_t)n * 4;
-  const size_t b_slot = multi ? (size_t)n_slots * 4 : 0, b_tv = multi ? tile_var.size() * 4 : 0;
-  if ((rc = ensure_pinned(h, c, b_t + b_v + b_b + 3 * b_i + b_slot + b_tv + 16))) return rc;
-  unsigned char* p_time = c->h_pin;
-  unsigned char* p = c->h_pin + b_t;
-  double* p_v = (double*)p;
-  double* p_b = (double*)(p + b_v);
-  int32_t* p_s = (int32_t*)(p + b_v + b_b);
-  int32_t* p_e = p_s + n;
-  int32_t* p_t = p_e + n;
-  int32_t* p_slot = p_t + n;
-  int32_t* p_tv = p_slot + (multi ? n_slots : 0);
-  int32_t* p_flag = p_tv + (multi ? tile_var.size() : 0);
-  host_copies({{p_time, t, b_t},
-               {p_v, vec6, b_v},
-               {p_b, beta, b_b},
-               {p_s, state, b_i},
-               {p_e, ixe, b_i},
-               {p_t, ixt, ixt ? b_i : 0},
-               {p_slot, slot_map.data(), b_slot},
-               {p_tv, tile_var.data(), b_tv}});
-  int32_t* d_state = c->d_i32;
-  int32_t* d_ixe = d_state + c->cap;
-  int32_t* d_ixt = d_ixe + c->cap;
-  int32_t* d_slot = d_ixt + c->cap;
-  int32_t* d_tvar = d_slot + c->cap_slots;
-  if (t) CU(h, cudaMemcpyAsync(c->d_t, p_time, b_t, cudaMemcpyHostToDevice, st));
-  CU(h, cudaMemcpy2DAsync(c->d_vec6, c->cap * 8, p_v, n * 8, n * 8, 6, cudaMemcpyHostToDevice, st));
-  CU(h, cudaMemcpyAsync(c->d_beta, p_b, b_b, cudaMemcpyHostToDevice, st));
-  CU(h, cudaMemcpyAsync(d_state, p_s, b_i, cudaMemcpyHostToDevice, st));
-  CU(h, cudaMemcpyAsync(d_ixe, p_e, b_i, cudaMemcpyHostToDevice, st));
-  if (ixt) CU(h, cudaMemcpyAsync(d_ixt, p_t, b_i, cudaMemcpyHostToDevice, st));
-  if (multi) {
-    CU(h, cudaMemcpyAsync(d_slot, p_slot, b_slot, cudaMemcpyHostToDevice, st));
-    CU(h, cudaMemcpyAsync(d_tvar, p_tv, b_tv, cudaMemcpyHostToDevice, st));
-  }
-  rc = track_device_impl(h, tun, c, nullptr, c->d_vec6, c->cap, c->d_beta, t ? c->d_t : nullptr, d_state, d_ixe,
-                         ixt ? d_ixt : nullptr,
-                         multi ? d_slot : nullptr, multi ? d_tvar : nullptr, n, n_slots, turn0, n_turns, rec_begin,
-                         rec_end, st);
+  const StageLayout Y(n, multi ? n_slots : 0, multi ? (int64_t)tile_var.size() : 0, t != nullptr);
+  if ((rc = ensure_staging(h, c, Y.bytes)) || (rc = ensure_pinned(h, c, Y.bytes))) return rc;
+  unsigned char *p = c->h_pin, *d = c->d_stage;
+  const size_t b_t = t ? (size_t)n * 16 : 0, b_v = (size_t)n * 48, b_b = (size_t)n * 8, b_i = (size_t)n * 4;
+  memset(p + Y.scratch, 0, 16);
+  host_copies({{p + Y.t, t, b_t},
+               {p + Y.vec6, vec6, b_v},
+               {p + Y.beta, beta, b_b},
+               {p + Y.state, state, b_i},
+               {p + Y.ixe, ixe, b_i},
+               {p + Y.ixt, ixt, ixt ? b_i : 0},
+               {p + Y.slot, slot_map.data(), multi ? (size_t)n_slots * 4 : 0},
+               {p + Y.tvar, tile_var.data(), multi ? tile_var.size() * 4 : 0}});
+  CU(h, cudaMemcpyAsync(d, p, Y.bytes, cudaMemcpyHostToDevice, st));
+  rc = track_device_impl(h, tun, at<int32_t>(d, Y.scratch), true, nullptr, at<double>(d, Y.vec6), n,
+                         at<double>(d, Y.beta), t ? at<uint64_t>(d, Y.t) : nullptr, at<int32_t>(d, Y.state),
+                         at<int32_t>(d, Y.ixe), ixt ? at<int32_t>(d, Y.ixt) : nullptr,
+                         multi ? at<int32_t>(d, Y.slot) : nullptr, multi ? at<int32_t>(d, Y.tvar) : nullptr, n,
+                         n_slots, turn0, n_turns, rec_begin, rec_end, st);
   if (rc) {
     cudaStreamSynchronize(st);
     return rc;
   }
-  CU(h, cudaMemcpyAsync(p_flag, c->d_scratch + 1, 4, cudaMemcpyDeviceToHost, st));
-  if (t) CU(h, cudaMemcpyAsync(p_time, c->d_t, b_t, cudaMemcpyDeviceToHost, st));
-  CU(h, cudaMemcpy2DAsync(p_v, n * 8, c->d_vec6, c->cap * 8, n * 8, 6, cudaMemcpyDeviceToHost, st));
-  CU(h, cudaMemcpyAsync(p_b, c->d_beta, b_b, cudaMemcpyDeviceToHost, st));
-  CU(h, cudaMemcpyAsync(p_s, d_state, b_i, cudaMemcpyDeviceToHost, st));
-  CU(h, cudaMemcpyAsync(p_e, d_ixe, b_i, cudaMemcpyDeviceToHost, st));
-  if (ixt) CU(h, cudaMemcpyAsync(p_t, d_ixt, b_i, cudaMemcpyDeviceToHost, st));
+  CU(h, cudaMemcpyAsync(p, d, Y.scratch + 16, cudaMemcpyDeviceToHost, st));
   CU(h, cudaStreamSynchronize(st));
-  if (*p_flag) return set_err(h, BGT_ETIMEOUT, "element-table staging did not complete");
-  host_copies({{t, p_time, b_t},
-               {vec6, p_v, b_v},
-               {beta, p_b, b_b},
-               {state, p_s, b_i},
-               {ixe, p_e, b_i},
-               {ixt, p_t, ixt ? b_i : 0}});
+  if (at<int32_t>(p, Y.scratch)[1]) return set_err(h, BGT_ETIMEOUT, "element-table staging did not complete");
+  host_copies({{t, p + Y.t, b_t},
+               {vec6, p + Y.vec6, b_v},
+               {beta, p + Y.beta, b_b},
+               {state, p + Y.state, b_i},
+               {ixe, p + Y.ixe, b_i},
+               {ixt, p + Y.ixt, ixt ? b_i : 0}});
   return 0;
 }
 
@@ -959,12 +945,16 @@ int bgt_da_scan_grid(bgt_handle* h, const double* ref_orbit, int32_t n_variants_
   cudaStream_t st = c->st;
   CU(h, L.use(st));
   const bool with_t = h->G.abs_time != 0;
-  if ((rc = ensure_staging(h, c, n, n_slots, n_tiles, with_t))) return rc;
-  int32_t* d_state = c->d_i32;
-  int32_t* d_ixe = d_state + c->cap;
-  int32_t* d_ixt = d_ixe + c->cap;
-  int32_t* d_slot = d_ixt + c->cap;
-  int32_t* d_tvar = d_slot + c->cap_slots;
+  const StageLayout Y(n, n_slots, n_tiles, with_t);
+  if ((rc = ensure_staging(h, c, Y.bytes))) return rc;
+  unsigned char* d = c->d_stage;
+  double* d_vec6 = at<double>(d, Y.vec6);
+  double* d_beta = at<double>(d, Y.beta);
+  int32_t* d_state = at<int32_t>(d, Y.state);
+  int32_t* d_ixe = at<int32_t>(d, Y.ixe);
+  int32_t* d_ixt = at<int32_t>(d, Y.ixt);
+  int32_t* d_slot = at<int32_t>(d, Y.slot);
+  int32_t* d_tvar = at<int32_t>(d, Y.tvar);
   int64_t n_rays = (int64_t)n_variants_used * n_delta * n_angle;
   // ray directions: angle_j = j * delta_angle + min_angle
   // (dynamic_aperture_mod.f90:88-95), cos/sin by the host C library
@@ -997,19 +987,19 @@ int bgt_da_scan_grid(bgt_handle* h, const double* ref_orbit, int32_t n_variants_
   CU(h, cudaMemsetAsync(d_slot, 0xff, (size_t)n_slots * 4, st));
   A.cs = d_cs;
   A.ref = d_ref;
-  A.vec6 = c->d_vec6;
-  A.stride = c->cap;
-  A.beta = c->d_beta;
+  A.vec6 = d_vec6;
+  A.stride = n;
+  A.beta = d_beta;
   A.state = d_state;
   A.ixe = d_ixe;
   A.ixt = d_ixt;
   A.slot = d_slot;
-  A.t = with_t ? c->d_t : nullptr;
+  A.t = with_t ? at<uint64_t>(d, Y.t) : nullptr;
   A.block = block;
   da_init_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A, n);
   da_tile_var_kernel<<<(unsigned)((n_tiles + 255) / 256), 256, 0, st>>>(d_tvar, tiles_per_var, n_tiles);
   h->launches += 2;
-  rc = track_device_impl(h, tun, c, nullptr, c->d_vec6, c->cap, c->d_beta, A.t, d_state, d_ixe, d_ixt, d_slot,
+  rc = track_device_impl(h, tun, c->d_scratch, false, nullptr, d_vec6, n, d_beta, A.t, d_state, d_ixe, d_ixt, d_slot,
                          d_tvar, n, n_slots, 0, n_turns, 0, h->n_ele, st);
   if (rc) return rc;
   da_reduce_kernel<<<(unsigned)((n_rays + 127) / 128), 128, 0, st>>>(d_state, d_ixt, n_rays, n_radius, A.dr, 0,
