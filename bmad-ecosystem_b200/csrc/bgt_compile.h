@@ -916,6 +916,24 @@ static int compile_element(const bgt_element& e, const bgt_species& sp, double p
   return 0;
 }
 
+// Set F_THEN_DRIFT on the records of a table (n_ele sequence entries) that
+// allow it and whose every use is followed by such a drift: records are
+// shared by identical elements, and none is added for the flag.
+static void mark_then_drift(double* tab, int32_t n_ele) {
+  const int32_t* seq = reinterpret_cast<const int32_t*>(tab);
+  auto hdr = [&](int e) { return reinterpret_cast<RecHdr*>(tab + seq[2 * e]); };
+  auto allowed = [&](int e) {
+    const RecHdr* h = hdr(e);
+    if (!(h->flags & F_NEAR) || h->kind == K_DRIFT || e + 1 == n_ele) return false;
+    const RecHdr* d = hdr(e + 1);
+    return d->kind == K_DRIFT && (d->flags & F_NEAR) && !(d->flags & (F_AP_ENTRANCE | F_AP_EXIT));
+  };
+  for (int e = 0; e < n_ele; e++)
+    if (allowed(e)) hdr(e)->flags |= F_THEN_DRIFT;
+  for (int e = 0; e < n_ele; e++)
+    if (!allowed(e)) hdr(e)->flags &= ~F_THEN_DRIFT;
+}
+
 // c_multi table, bmad/low_level/c_multi.f90:19-75
 static void c_multi_tables(double cm[BGT_MAXPOLE_DEV + 1][BGT_MAXPOLE_DEV + 1],
                            double cm0[BGT_MAXPOLE_DEV + 1][BGT_MAXPOLE_DEV + 1]) {
@@ -1008,6 +1026,7 @@ static int compile_tables(const bgt_element* eles, int32_t n_ele, int32_t n_vari
       s[0] = off;
       s[1] = eles[(int64_t)v * n_ele + e].ix_ele;
     }
+    mark_then_drift(tab.data(), n_ele);
     table_dw = std::max(table_dw, (int32_t)tab.size());
     table_off.push_back((int64_t)all.size());
     all.insert(all.end(), tab.begin(), tab.end());

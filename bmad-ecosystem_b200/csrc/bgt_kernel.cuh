@@ -690,7 +690,8 @@ namespace bgt {
 struct GeneralCall {
   Part p;
   const Glob* G;
-  double a, r_pc;  // the memo of pz (TODO_BODY)
+  double a, r_pc;      // the memo of pz (TODO_BODY)
+  const double* then;  // the drift record to take along, or nullptr; cleared when it is reached
 };
 template <bool RARE>
 BGT_DEV_NOINLINE void track1_general(GeneralCall* io, const double* rec, QMemo qm, int todo) {
@@ -707,6 +708,7 @@ BGT_DEV_NOINLINE void track1_general(GeneralCall* io, const double* rec, QMemo q
   Rec R = decode<RARE>(rec);
   const int32_t fl = R.h->flags;
   int32_t kind = R.h->kind;
+  bool near_body = false;
   if (todo == TODO_EXIT) {
     kind = K_MARKER;
   } else if (todo == TODO_BODY) {  // the entrance aperture is passed
@@ -715,6 +717,7 @@ BGT_DEV_NOINLINE void track1_general(GeneralCall* io, const double* rec, QMemo q
     if (body_near(p, R.h, R.mis, R.kb, G.mal, io->a, io->r_pc, qm)) {
       if (RARE) element_exit_time(p, t0, z0, R.kb[kind == K_QUAD ? Q_DTREF : TM_DTREF], G);
       kind = K_MARKER;
+      near_body = true;
     }
   } else if ((fl & F_AP_ENTRANCE) && G.ap_on) {
     if (RARE)
@@ -753,13 +756,22 @@ BGT_DEV_NOINLINE void track1_general(GeneralCall* io, const double* rec, QMemo q
     else
       aperture_limits(p, R.ap, fl, p.x, p.y);
   }
+  if (io->then && p.state == ALIVE) {
+    const double* then = io->then;
+    io->then = nullptr;
+    if (near_body && abs_hi(p.px) < NEAR_P_HI && abs_hi(p.py) < NEAR_P_HI)
+      drift_record_near<RARE>(p, then, G, io->a, io->r_pc);
+    else
+      track_a_drift<true>(p, then[HDR_DW + DR_L], G, m);
+    orbit_too_large(p, G);
+  }
 }
 
-// What track1_near left to do
+// What track1_near left to do; true when the drift `then` was reached
 template <bool RARE>
-__device__ __forceinline__ void track1_rest(Part& p, const double* rec, const Glob& G, DriftMemo& m, QMemo qm,
-                                            int todo) {
-  GeneralCall io = {p, &G, m.a, m.r_pc};
+__device__ __forceinline__ bool track1_rest(Part& p, const double* rec, const double* then, const Glob& G,
+                                            DriftMemo& m, QMemo qm, int todo) {
+  GeneralCall io = {p, &G, m.a, m.r_pc, then};
   track1_general<RARE>(&io, rec, qm, todo);
   const uint64_t t_lo = p.t_lo, t_hi = p.t_hi;
   p = io.p;
@@ -767,12 +779,14 @@ __device__ __forceinline__ void track1_rest(Part& p, const double* rec, const Gl
     p.t_lo = t_lo;
     p.t_hi = t_hi;
   }
+  return then && !io.then;
 }
 
 template <bool RARE>
 __device__ __forceinline__ void track1_rec(Part& p, const double* rec, const Glob& G, DriftMemo& m, QMemo qm) {
-  const int todo = track1_near<RARE>(p, rec, G, m, qm);
-  if (todo != TODO_NOTHING) track1_rest<RARE>(p, rec, G, m, qm, todo);
+  const int32_t fl = reinterpret_cast<const RecHdr*>(rec)->flags;
+  const int todo = track1_near<RARE>(p, rec, fl, nullptr, G, m, qm);
+  if (todo != TODO_NOTHING) track1_rest<RARE>(p, rec, nullptr, G, m, qm, todo);
 }
 
 #ifdef __CUDACC__
@@ -788,13 +802,20 @@ __device__ __forceinline__ void track_warp_turn(Part& p, int32_t& ixe, int32_t& 
                                                 DriftMemo& m, QMemo qm) {
   for (int r = begin; r < end; r++) {
     const int2 e = seq[r];
+    const double* rec = table + e.x;
+    const int32_t fl = reinterpret_cast<const RecHdr*>(rec)->flags;
+    const double* then = nullptr;
+    if ((fl & F_THEN_DRIFT) && r + 1 < end) then = table + seq[++r].x;
     int todo = TODO_NOTHING;
-    if (p.state == ALIVE) todo = track1_near<RARE>(p, table + e.x, G, m, qm);
+    if (p.state == ALIVE) todo = track1_near<RARE>(p, rec, fl, then, G, m, qm);
     if (__any_sync(0xffffffffu, todo != TODO_NOTHING)) {
       if (todo != TODO_NOTHING) {
-        track1_rest<RARE>(p, table + e.x, G, m, qm, todo);
+        const bool in_drift = todo == TODO_DRIFT_EXIT;
+        const bool drift = track1_rest<RARE>(p, in_drift ? then : rec, in_drift ? nullptr : then, G, m, qm,
+                                             in_drift ? (int)TODO_EXIT : todo) ||
+                           in_drift;
         if (p.state != ALIVE) {
-          ixe = e.y;
+          ixe = drift ? seq[r].y : e.y;
           ixt = turn;
         }
       }

@@ -89,6 +89,9 @@ enum Flag : int32_t {
   // quadrupole or thick multipole with magnetic multipoles up to order 7 and
   // offsets and roll at most; lab-frame apertures without momentum limits
   F_NEAR = 1 << 30,
+  // the record has a near-axis form other than a drift's, and the next one of
+  // the sequence is a drift without apertures, which that form takes along
+  F_THEN_DRIFT = INT32_MIN,
 };
 
 struct alignas(8) RecHdr {

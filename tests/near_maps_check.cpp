@@ -37,7 +37,7 @@ static double logu(double a, double b) { return exp(uni(log(a), log(b))); }
 static double sign() { return (rng() & 1) ? 1.0 : -1.0; }
 
 struct Count {
-  const char* name;
+  std::string name;
   long bad = 0, passed = 0, total = 0;
   void add(bool test_held, bool equal) {
     total++;
@@ -45,7 +45,7 @@ struct Count {
     passed++;
     if (!equal) bad++;
   }
-  ~Count() { printf("%s %ld %ld %ld\n", name, bad, passed, total); }
+  ~Count() { printf("%s %ld %ld %ld\n", name.c_str(), bad, passed, total); }
 };
 
 static void math_checks(long n) {
@@ -139,7 +139,9 @@ static bgt_element element(int key, double l) {
 
 static bool same(double a, double b) { return a == b || (a != a && b != b); }
 
-static void one_form(const char* name, bgt_element e, long n) {
+// One record form alone (then = false), and with the drift that follows it
+// taken along (then = true), against the general maps one record at a time.
+static void one_form(const std::string& name, bgt_element e, long n, bool then) {
   bgt_species sp;
   memset(&sp, 0, sizeof(sp));
   sp.mass = MASS;
@@ -151,12 +153,17 @@ static void one_form(const char* name, bgt_element e, long n) {
   int32_t dw = 0;
   bool rare = false;
   std::string msg;
-  Count c{name};
-  if (host::compile_tables(&e, 1, 1, sp, QMEMO_CLASSES, all, off, dw, rare, msg) || rare) {
+  Count c{name + (then ? "+drift" : "")};
+  const bgt_element eles[2] = {e, element(BGT_DRIFT, 0.3)};
+  if (host::compile_tables(eles, then ? 2 : 1, 1, sp, QMEMO_CLASSES, all, off, dw, rare, msg) || rare) {
     c.bad = -1;
     return;
   }
-  const double* rec = all.data() + off[0] + *reinterpret_cast<const int32_t*>(all.data() + off[0]);
+  const double* tab = all.data() + off[0];
+  const int32_t* seq = reinterpret_cast<const int32_t*>(tab);
+  const double *rec = tab + seq[0], *next = then ? tab + seq[2] : nullptr;
+  const int32_t fl = reinterpret_cast<const RecHdr*>(rec)->flags;
+  if (then != ((fl & F_THEN_DRIFT) != 0)) c.bad = -1;
   Glob G{};
   G.mc2 = MASS;
   G.mc2sq = MASS * MASS;
@@ -186,21 +193,29 @@ static void one_form(const char* name, bgt_element e, long n) {
     Part a = p;
     DriftMemo m;
     m.pz = NAN;
-    const int todo = track1_near<false>(a, rec, G, m, QMemo{qa, 1});
-    GeneralCall io = {p, &G, 0, 0};
-    track1_general<false>(&io, rec, QMemo{qb, 1}, TODO_ALL);
-    if (todo != TODO_NOTHING) {  // what is left to do out of line gives the same
-      GeneralCall rest = {a, &G, m.a, m.r_pc};
-      track1_general<false>(&rest, rec, QMemo{qa, 1}, todo);
-      a = rest.p;
+    const int todo = track1_near<false>(a, rec, fl, next, G, m, QMemo{qa, 1});
+    bool a_drift = next && todo == TODO_NOTHING;  // the particle is past the element
+    if (todo != TODO_NOTHING) {  // as track_warp_turn
+      const bool in_drift = todo == TODO_DRIFT_EXIT;
+      a_drift = track1_rest<false>(a, in_drift ? next : rec, in_drift ? nullptr : next, G, m, QMemo{qa, 1},
+                                   in_drift ? (int)TODO_EXIT : todo) ||
+                in_drift;
     }
+    GeneralCall io = {p, &G, 0, 0, nullptr};
+    track1_general<false>(&io, rec, QMemo{qb, 1}, TODO_ALL);
+    const bool b_drift = next && io.p.state == ALIVE;
+    if (b_drift) track1_general<false>(&io, next, QMemo{qb, 1}, TODO_ALL);
     const Part& b = io.p;
     const bool equal = same(a.x, b.x) && same(a.px, b.px) && same(a.y, b.y) && same(a.py, b.py) && same(a.z, b.z) &&
-                       a.pz == b.pz && a.beta == b.beta && a.state == b.state;
+                       a.pz == b.pz && a.beta == b.beta && a.state == b.state && a_drift == b_drift;
     c.total++;
     if (todo == TODO_NOTHING || todo == TODO_BODY) c.passed++;
     if (!equal) c.bad++;
   }
+}
+static void one_form(const std::string& name, bgt_element e, long n) {
+  one_form(name, e, n, false);
+  if (e.key != BGT_DRIFT) one_form(name, e, n, true);
 }
 
 static void map_checks(long n) {
@@ -237,7 +252,7 @@ static void map_checks(long n) {
       q.an[k] += pow(100.0, k - 1) * 1e-4;
       if (k != 1) q.bn[k] = -pow(100.0, k - 1) * 2e-4;
       if (k > 3) q.bn[k - 2] += pow(100.0, k - 3) * 1e-4;
-      one_form(("quad_errors_" + std::to_string(k)).c_str(), q, n);
+      one_form("quad_errors_" + std::to_string(k), q, n);
     }
   }
   bgt_element s = element(BGT_SEXTUPOLE, 0.2);

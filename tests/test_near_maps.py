@@ -8,7 +8,8 @@ test holds (which it must for all but 1 in 1000 arguments), the maps with the
 general maps on particles inside, at and outside the near-axis region, on
 axis, past apertures and limits, for every record form that has a near-axis
 form (multipole orders 0 to 7, offsets and roll, both apertures at both ends,
-zero and negative lengths, edges at one end, bend angles up to the limit).
+zero and negative lengths, edges at one end, bend angles up to the limit),
+alone and with the drift that follows taken along.
 """
 from __future__ import annotations
 
@@ -50,7 +51,7 @@ def test_arithmetic_is_correctly_rounded(checker, seed):
 @pytest.mark.parametrize("seed", [1, 2])
 def test_near_axis_maps_equal_the_general_maps(checker, seed):
     rows = run(checker, "maps", 8000, seed)
-    assert len(rows) == 43
+    assert len(rows) == 82
     for name, bad, passed, total in rows:
         assert bad == 0, name
         assert 0.2 * total < passed < 0.9 * total, name  # both sides of the region's edge are covered
