@@ -440,7 +440,6 @@ def run_learned_da(args):
     with ClockSampler(R.local) as clk:
         jit = (None, args.seed) if args.jitter else (None,)
         pb_tr, scans, train_scan_s = _staged_scan_sharded(R, lats, rings.CONFIG2_GRID, turns, half, jit, tun)
-        # 65,536-row inference chunks: several tiles per CTA in each GEMM launch
         net = SurvivalMLP(max_batch=65536, seed=args.seed)
         train = _train_classifier(args, R, pb_tr, scans, net)
         R.barrier()
@@ -589,8 +588,8 @@ def run_sext_scan(args):
 
 def run_mlp(args):
     """The survival classifier on its own: one step = 200 forward passes over
-    --mlp-rows probes each (three tcgen05 GEMM layers and the output head, in
-    65,536-row chunks; 200 passes so the clock sampler sees the timed region)
+    --mlp-rows probes each (three tcgen05 layers and the output layer in one
+    kernel; 200 passes so the clock sampler sees the timed region)
     and, separately, 200 Adam training steps on an 8,192-sample batch; CUDA
     events on the launching stream.  Beside it the same three layers as torch
     bf16 matmuls (cuBLAS) with ReLU, for context."""
@@ -649,7 +648,7 @@ def run_mlp(args):
             "value": tf, "unit": "TFLOP/s", "higher_is_better": True, "n_gpus": 1, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_fwd * passes, "ms_per_forward": ms_fwd, "dtype": "bf16",
             "data": "synthetic",
-            "config": {"workload": "64-256-256-256-1 MLP forward", "rows": rows, "chunk_rows": 65536,
+            "config": {"workload": "64-256-256-256-1 MLP forward", "rows": rows,
                        "passes_per_step": passes},
             "roofline": {"bound": "tensor", "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak,
                          "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst)" if peaks else "fallback"},
