@@ -372,6 +372,7 @@ static bool record_has_near(const double* rec, const RecHdr& h) {
   const double* mis = rec + HDR_DW;
   const double* q = mis + ((fl & F_MISALIGN) ? MIS_N : 0) + ((fl & (F_AP_ENTRANCE | F_AP_EXIT)) ? AP_N : 0);
   switch (h.kind) {
+    case K_MARKER:
     case K_DRIFT:
       return !(fl & F_MISALIGN);
     case K_BEND:

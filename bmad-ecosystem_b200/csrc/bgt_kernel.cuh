@@ -13,8 +13,9 @@
 // block prefix sum through shared memory) so dead lanes stop costing issue
 // slots; fully dead warps skip the element loop.
 //
-// An element's map is its near-axis form where the particle allows it
-// (bgt_near.cuh), else the general map, out of line.
+// An element's map is its near-axis form where the record has one and the
+// particle allows it (bgt_near.cuh), else the general map, in a loop of its
+// own (track_warp_turn).
 //
 // Everything up to track1_rec is per-particle arithmetic with no CUDA
 // construct beyond the __device__ qualifiers; a plain C++ compiler that
@@ -678,55 +679,23 @@ __device__ __forceinline__ void body_bend(Part& p, const Rec& R, const Glob& G, 
 
 namespace bgt {
 
-// track1, bmad/code/track1.f90:43-342 for one alive particle and one record:
-// entrance aperture, body, orbit_too_large, exit aperture.  Returns the
-// particle with its state (ALIVE or a lost code).  Out of line: in a ring
-// only the RF cavity and the particles near a limit come here, and inlined
-// it would put its code and its register demand into the element loop.  The
-// memo of pz is its own (the caller's stays valid by its key).
-// todo: what is left to do (NearTodo).  The particle goes through memory:
-// passed and returned by value it would tie the element loop's registers to
-// the calling convention.
-struct GeneralCall {
-  Part p;
-  const Glob* G;
-  double a, r_pc;      // the memo of pz (TODO_BODY)
-  const double* then;  // the drift record to take along, or nullptr; cleared when it is reached
-};
+// track1, bmad/code/track1.f90:43-342 for one alive particle and one record
+// by the general maps: entrance aperture, body, orbit_too_large, exit
+// aperture.  p.state is ALIVE or a lost code afterwards.
 template <bool RARE>
-BGT_DEV_NOINLINE void track1_general(GeneralCall* io, const double* rec, QMemo qm, int todo) {
-  Part p = io->p;
-  Glob G = *io->G;
+__device__ __forceinline__ void track1_all(Part& p, const double* rec, const Glob& glob, DriftMemo& m, QMemo qm) {
+  Glob G = glob;
   if (!RARE) G.track_time = 0;  // no particle time in these instances
-  struct Store {
-    GeneralCall* io;
-    const Part& p;
-    __device__ __forceinline__ ~Store() { io->p = p; }
-  } store{io, p};
-  DriftMemo m;
-  m.pz = NAN;
   Rec R = decode<RARE>(rec);
   const int32_t fl = R.h->flags;
-  int32_t kind = R.h->kind;
-  bool near_body = false;
-  if (todo == TODO_EXIT) {
-    kind = K_MARKER;
-  } else if (todo == TODO_BODY) {  // the entrance aperture is passed
-    const qp::Q t0 = time_of(p);
-    const double z0 = p.z;
-    if (body_near(p, R.h, R.mis, R.kb, G.mal, io->a, io->r_pc, qm)) {
-      if (RARE) element_exit_time(p, t0, z0, R.kb[kind == K_QUAD ? Q_DTREF : TM_DTREF], G);
-      kind = K_MARKER;
-      near_body = true;
-    }
-  } else if ((fl & F_AP_ENTRANCE) && G.ap_on) {
+  if ((fl & F_AP_ENTRANCE) && G.ap_on) {
     if (RARE)
       check_aperture(p, R.ap, R.mis, fl, false);
     else
       aperture_limits(p, R.ap, fl, p.x, p.y);
     if (p.state != ALIVE) return;
   }
-  switch (kind) {
+  switch (R.h->kind) {
     case K_DRIFT:
       track_a_drift<true>(p, R.kb[DR_L], G, m);
       break;
@@ -756,30 +725,52 @@ BGT_DEV_NOINLINE void track1_general(GeneralCall* io, const double* rec, QMemo q
     else
       aperture_limits(p, R.ap, fl, p.x, p.y);
   }
-  if (io->then && p.state == ALIVE) {
-    const double* then = io->then;
-    io->then = nullptr;
-    if (near_body && abs_hi(p.px) < NEAR_P_HI && abs_hi(p.py) < NEAR_P_HI)
-      drift_record_near<RARE>(p, then, G, io->a, io->r_pc);
-    else
-      track_a_drift<true>(p, then[HDR_DW + DR_L], G, m);
-    orbit_too_large(p, G);
-  }
 }
 
-// What track1_near left to do; true when the drift `then` was reached
+// What track1_near left (todo) of a record, and of the drift `then` after it,
+// as far as the near-axis forms go: body_near and the checks that may lose the
+// particle (a F_NEAR record's apertures are in the lab frame).  Returns how
+// many of the two are done; the rest is the general maps'.  A particle lost
+// here is lost in the record that is not done.
+template <bool RARE>
+__device__ __forceinline__ int track1_finish(Part& p, const double* rec, const double* then, const Glob& G,
+                                             const DriftMemo& m, QMemo qm, int todo) {
+  if (todo == TODO_ALL) return 0;
+  if (todo != TODO_DRIFT_EXIT) {
+    const RecHdr* h = reinterpret_cast<const RecHdr*>(rec);
+    const int32_t fl = h->flags;
+    const double* mis = rec + HDR_DW;
+    const double* ap = mis + ((fl & F_MISALIGN) ? MIS_N : 0);
+    if (todo == TODO_BODY) {
+      if (!(h->poles & ~3)) return 0;  // short: the general map costs no more
+      const double* q = ap + ((fl & (F_AP_ENTRANCE | F_AP_EXIT)) ? AP_N : 0);
+      const qp::Q t0 = time_of(p);
+      const double z0 = p.z;
+      if (!body_near(p, h, mis, q, G.mal, m.a, m.r_pc, qm)) return 0;
+      if (RARE) element_exit_time(p, t0, z0, q[h->kind == K_QUAD ? Q_DTREF : TM_DTREF], G);
+    }
+    if (orbit_too_large(p, G)) return 0;
+    if ((fl & F_AP_EXIT) && G.ap_on) aperture_limits(p, ap, fl, p.x, p.y);
+    if (p.state != ALIVE) return 0;
+    if (!then || !(abs_hi(p.px) < m.near_p && abs_hi(p.py) < m.near_p)) return 1;
+    drift_record_near<RARE>(p, then, G, m.a, m.r_pc);
+  }
+  return orbit_too_large(p, G) ? 1 : 2;
+}
+
+// The rest of a record, and of the drift `then`, for one particle on its own;
+// true when the drift was reached
 template <bool RARE>
 __device__ __forceinline__ bool track1_rest(Part& p, const double* rec, const double* then, const Glob& G,
                                             DriftMemo& m, QMemo qm, int todo) {
-  GeneralCall io = {p, &G, m.a, m.r_pc, then};
-  track1_general<RARE>(&io, rec, qm, todo);
-  const uint64_t t_lo = p.t_lo, t_hi = p.t_hi;
-  p = io.p;
-  if (!RARE) {  // no particle time in these instances
-    p.t_lo = t_lo;
-    p.t_hi = t_hi;
+  int done = track1_finish<RARE>(p, rec, then, G, m, qm, todo);
+  if (done == 0 && p.state == ALIVE) {
+    track1_all<RARE>(p, rec, G, m, qm);
+    done = 1;
+    if (p.state != ALIVE) return false;
   }
-  return then && !io.then;
+  if (then && done == 1 && p.state == ALIVE) track1_all<RARE>(p, then, G, m, qm);
+  return then && done > 0;
 }
 
 template <bool RARE>
@@ -789,37 +780,93 @@ __device__ __forceinline__ void track1_rec(Part& p, const double* rec, const Glo
   if (todo != TODO_NOTHING) track1_rest<RARE>(p, rec, nullptr, G, m, qm, todo);
 }
 
-#ifdef __CUDACC__
-// One turn of a warp's particles through the records [begin, end).  Every
-// lane stays in the loop and votes after each near-axis map, so that the warp
-// is whole again before the next element: without the vote a lane that took
-// the general maps once runs apart from its warp for the rest of the turn,
-// and the warp issues everything twice (absolute-time tracking: 4.2 ms
-// instead of 1.2 for 40,000 particle turns).
+#ifndef __CUDACC__
+// A record by the general maps alone: what the host programs compare the
+// near-axis forms with
+struct GeneralCall {
+  Part p;
+  const Glob* G;
+  double a, r_pc;      // unused: the memo of pz is the call's own
+  const double* then;  // unused
+};
+template <bool RARE>
+void track1_general(GeneralCall* io, const double* rec, QMemo qm, int) {
+  DriftMemo m;
+  m.pz = NAN;
+  track1_all<RARE>(io->p, rec, *io->G, m, qm);
+}
+#else
+// One turn of a warp's particles through the records [begin, end): a loop of
+// near-axis forms and a loop of general maps, one after the other.
+//
+// Every lane stays in the loop it is in and votes after each near-axis map, so
+// that the warp is whole again before the next element: without the vote a
+// lane that took the general maps once runs apart from its warp for the rest
+// of the turn, and the warp issues everything twice (absolute-time tracking:
+// 4.2 ms instead of 1.2 for 40,000 particle turns).
+//
+// Two loops, not one: within one loop the general maps' registers cost the
+// near-axis forms their interleaving (a drift 13 spill loads instead of 6),
+// and out of line a call stored and reloaded 70 registers, 9 KB a warp, which
+// local memory writes through to L2: 606,208 particles x 16 elements took
+// 0.38 ms of markers, 0.46 of kickers, 0.81 of rbends, and 0.43 of drifts for
+// particles outside the near-axis region.  Side by side the register sets are
+// separate: 0.07, 0.13, 0.58 and 0.16 ms (with the general maps alone, before
+// there were near-axis forms: 0.08, 0.20, 0.57, 0.14).
+//
+// The warp leaves the general loop at a record whose near-axis form pays for
+// the change (a bend, or a magnet with a sextupole or higher order), when all
+// its particles are a factor of two inside the region, so that one on the edge
+// does not change loops at every magnet; drifts and plain quadrupoles until
+// there cost about the same by either.
 template <bool RARE>
 __device__ __forceinline__ void track_warp_turn(Part& p, int32_t& ixe, int32_t& ixt, const int2* seq,
                                                 const double* table, int begin, int end, int turn, const Glob& G,
                                                 DriftMemo& m, QMemo qm) {
-  for (int r = begin; r < end; r++) {
-    const int2 e = seq[r];
-    const double* rec = table + e.x;
-    const int32_t fl = reinterpret_cast<const RecHdr*>(rec)->flags;
-    const double* then = nullptr;
-    if ((fl & F_THEN_DRIFT) && r + 1 < end) then = table + seq[++r].x;
-    int todo = TODO_NOTHING;
-    if (p.state == ALIVE) todo = track1_near<RARE>(p, rec, fl, then, G, m, qm);
-    if (__any_sync(0xffffffffu, todo != TODO_NOTHING)) {
-      if (todo != TODO_NOTHING) {
-        const bool in_drift = todo == TODO_DRIFT_EXIT;
-        const bool drift = track1_rest<RARE>(p, in_drift ? then : rec, in_drift ? nullptr : then, G, m, qm,
-                                             in_drift ? (int)TODO_EXIT : todo) ||
-                           in_drift;
+  int r = begin;
+  while (r < end) {
+    int at, todo;
+    const double *rec, *then;
+    bool any;
+    do {
+      at = r++;
+      rec = table + seq[at].x;
+      const int32_t fl = reinterpret_cast<const RecHdr*>(rec)->flags;
+      then = nullptr;
+      if ((fl & F_THEN_DRIFT) && r < end) then = table + seq[r++].x;
+      todo = TODO_NOTHING;
+      if (p.state == ALIVE) todo = track1_near<RARE>(p, rec, fl, then, G, m, qm);
+      any = __any_sync(0xffffffffu, todo != TODO_NOTHING);
+    } while (!any && r < end);
+    if (!any) break;
+    int mine = r;  // this lane's next record
+    if (todo != TODO_NOTHING) {
+      mine = at + track1_finish<RARE>(p, rec, then, G, m, qm, todo);
+      if (p.state != ALIVE) {
+        ixe = seq[mine].y;
+        ixt = turn;
+      }
+    }
+    if (!__any_sync(0xffffffffu, p.state == ALIVE && mine < r)) continue;
+    int i = at;
+    for (; i < end; i++) {
+      rec = table + seq[i].x;
+      const RecHdr* h = reinterpret_cast<const RecHdr*>(rec);
+      if ((h->flags & F_NEAR) && (h->kind == K_BEND || (h->poles & ~3)) && i >= r) {
+        drift_memo(p, G, m);
+        const int32_t lim = m.near_p - 0x00100000;  // half of the region
+        const bool near = abs_hi(p.px) < lim && abs_hi(p.py) < lim;
+        if (__all_sync(0xffffffffu, near || p.state != ALIVE)) break;
+      }
+      if (p.state == ALIVE && i >= mine) {
+        track1_all<RARE>(p, rec, G, m, qm);
         if (p.state != ALIVE) {
-          ixe = drift ? seq[r].y : e.y;
+          ixe = seq[i].y;
           ixt = turn;
         }
       }
     }
+    r = i;
   }
 }
 

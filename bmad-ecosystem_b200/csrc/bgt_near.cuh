@@ -5,7 +5,7 @@
 // of bgt_kernel.cuh need none of their range checks, lost-particle branches
 // and general quotients, and each element becomes one or a few basic blocks
 // inside the element loop; the general maps, which also decide every loss,
-// stay out of line.  All values are the general maps': the same operations
+// have a loop of their own.  All values are the general maps': the same operations
 // in the same order, quotients, square roots and transcendentals the IEEE
 // (correctly rounded) ones by bgt_fastmath.cuh.
 //
@@ -165,16 +165,26 @@ struct SparseKicks {
     c.py = c.py + ky;
   }
 };
+// Orders 0 or 2 alone, or none: kickers, plain sextupoles, and what has no field
+struct PlainKicks {
+  __device__ __forceinline__ static bool holds(int32_t poles) { return (poles & ~4) == 0 || poles == 1; }
+  __device__ __forceinline__ static void apply(Part& c, const double* an, const double* bn, int32_t poles,
+                                               double scale) {
+    if (poles == 4)
+      DenseKicks<2, 2>::apply(c, an, bn, poles, scale);
+    else if (poles == 1)
+      DenseKicks<0, 0>::apply(c, an, bn, poles, scale);
+  }
+};
 struct NoKicks {
   __device__ __forceinline__ static void apply(Part&, const double*, const double*, int32_t, double) {}
 };
 
-// f(kicks) for the orders of `poles`: none, dense from the sextupole or the
-// octupole up, else sparse
+// f(kicks) for the orders of `poles`: dense from the sextupole or the octupole
+// up, else sparse
 template <class F>
 __device__ __forceinline__ bool with_kicks(int32_t poles, const F& f) {
   switch (poles) {
-    case 0x00: return f(NoKicks{});
     case 0x04: return f(DenseKicks<2, 2>{});
     case 0x0c: return f(DenseKicks<2, 3>{});
     case 0x1c: return f(DenseKicks<2, 4>{});
@@ -232,8 +242,10 @@ __device__ __forceinline__ void quad_steps(Part& c, const QuadMats& M, double dz
   const double* an = q + Q_N;
   const double* bn = an + (h->ix_mag_max + 1);
   const double r_half = q[Q_RHALF], r_step = q[Q_RSTEP];
-  KICKS::apply(c, an, bn, poles, r_half);
-  for (int i = 1; i <= n_step; i++) {
+#pragma unroll 1
+  for (int i = 0;; i++) {
+    KICKS::apply(c, an, bn, poles, i == 0 || i == n_step ? r_half : r_step);
+    if (i >= n_step) break;
     const double x = c.x, px = c.px, y = c.y, py = c.py;
     c.z = c.z + (M.x.z0 * (x * x) + M.x.z1 * x * px + M.x.z2 * (px * px) + M.y.z0 * (y * y) + M.y.z1 * y * py +
                  M.y.z2 * (py * py));
@@ -242,7 +254,6 @@ __device__ __forceinline__ void quad_steps(Part& c, const QuadMats& M, double dz
     c.y = M.y.cx * y + M.y.m01 * py;
     c.py = M.y.m10 * y + M.y.cx * py;
     c.z = c.z + dz_low;
-    KICKS::apply(c, an, bn, poles, i == n_step ? r_half : r_step);
   }
 }
 
@@ -289,48 +300,60 @@ __device__ __forceinline__ bool thick_steps(Part& c, const RecHdr* h, const doub
   const double* bn = an + (h->ix_mag_max + 1);
   const double step = q[TM_STEP], rel_pc = 1 + c.pz;
   const double r_half = q[TM_RHALF], r_step = q[TM_RSTEP];
-  KICKS::apply(c, an, bn, poles, r_half);
-  for (int i = 1; i <= n_step; i++) {
+#pragma unroll 1
+  for (int i = 0;; i++) {
+    KICKS::apply(c, an, bn, poles, i == 0 || i == n_step ? r_half : r_step);
+    if (i >= n_step) break;
     if (!inside_limits(c.x, c.px, c.y, c.py, mal)) return false;
     if (step != 0) drift_near(c, step, rel_pc, a, r_pc);
-    KICKS::apply(c, an, bn, poles, i == n_step ? r_half : r_step);
   }
   return true;
 }
 
 // ---------------------------------------------------------------------------
-// The body of any F_NEAR quadrupole or thick multipole.  Called out of line
-// (track1_general) for the ones that are misaligned or carry multipoles other
-// than a sextupole's, and where a quadrupole's matrices are not in the memo,
-// so that the element loop holds the registers and the code of the plain ones
-// only; the call costs ~280 instructions, of 950 for a sextupole and 3800 for
-// a quadrupole of 16 steps (inlined, they raised every drift's spills from 6
-// loads to 13).  false, p unchanged, for the general maps: the exact
-// low-energy correction, or a particle that leaves the near-axis region on
-// the way (offset_particle then leaves its position as it is).
+// The body of a F_NEAR quadrupole or thick multipole with a sextupole or
+// higher order, misaligned or not: between the near-axis loop and the general
+// one (track_warp_turn), so that the near-axis loop holds the registers and
+// the code of the plain elements only (within it, they raised every drift's
+// spills from 6 loads to 13).  The change of place costs ~150 issue slots,
+// which a body with only orders 0 and 1 does not win back (606,208 particles x
+// 16 such magnets 0.33 ms, by the general maps 0.18): those go to the general
+// maps.  false, p unchanged, for the general maps too: the exact low-energy
+// correction, or a particle that leaves the near-axis region on the way
+// (offset_particle then leaves its position as it is).
+//
+// The kicks stand at one place in each of the loops over the steps, which are
+// not unrolled: a first half kick of its own before the loop doubles the code
+// (a kernel instance compiles in 55 s instead of 24), and a peeled first step
+// costs registers in the near-axis loop (10,000 particles x 16 turns of the
+// ring 6.5 -> 6.4 ms without).
 __device__ __forceinline__ bool body_near(Part& p, const RecHdr* h, const double* mis, const double* q, double mal,
                                           double a, double r_pc, QMemo qm) {
-  Part c = p;
   const int32_t fl = h->flags;
-  if (fl & F_MISALIGN) offset_near(c, mis, fl, true);
+  double dz_low;
+  if (h->kind == K_QUAD && !quad_low_energy(p.pz, q, dz_low)) return false;
+  Saved start(p);
+  if (fl & F_MISALIGN) offset_near(p, mis, fl, true);
   if (h->kind == K_QUAD) {
     QuadMats M;
-    double dz_low;
-    if (!quad_low_energy(c.pz, q, dz_low)) return false;
-    if (!quad_memo(1 + c.pz, h->aux0, qm, M)) quad_memo_fill(1 + c.pz, h->aux0, qm, q, M);
+    if (!quad_memo(1 + p.pz, h->aux0, qm, M)) quad_memo_fill(1 + p.pz, h->aux0, qm, q, M);
     with_kicks(h->poles, [&](auto kicks) {
-      quad_steps<decltype(kicks)>(c, M, dz_low, h, q);
+      quad_steps<decltype(kicks)>(p, M, dz_low, h, q);
       return true;
     });
   } else {
-    if (!with_kicks(h->poles, [&](auto kicks) { return thick_steps<decltype(kicks)>(c, h, q, mal, a, r_pc); }))
+    if (!with_kicks(h->poles, [&](auto kicks) { return thick_steps<decltype(kicks)>(p, h, q, mal, a, r_pc); })) {
+      start.restore(p);
       return false;
+    }
   }
   if (fl & F_MISALIGN) {
-    if (!(abs_hi(c.px) < NEAR_P_HI && abs_hi(c.py) < NEAR_P_HI)) return false;
-    offset_near(c, mis, fl, false);
+    if (!(abs_hi(p.px) < NEAR_P_HI && abs_hi(p.py) < NEAR_P_HI)) {
+      start.restore(p);
+      return false;
+    }
+    offset_near(p, mis, fl, false);
   }
-  p = c;
   return true;
 }
 
@@ -360,7 +383,8 @@ __device__ __forceinline__ void hwang_edge_normal(double& x, double px, double y
   }
 }
 
-// The exact sector body with edges normal to the orbit (BEND_PLAIN records):
+// The exact sector body with edges normal to the orbit (F_NEAR bends,
+// bend_is_plain in bgt_compile.h):
 // the arithmetic of body_bend's exact step, every rounded value the same, in
 // one basic block.  false where body_bend has to decide: a rounding test
 // that failed, an argument outside the light ranges, the near-axis
@@ -430,12 +454,12 @@ __device__ __forceinline__ bool bend_near(Part& p, const double* q, int32_t fl, 
 }
 
 // ---------------------------------------------------------------------------
-// track1 through a record by its near-axis form.  What is left to do out of
-// line (track1_general): TODO_NOTHING; TODO_EXIT, the checks after the body,
-// where the particle may be past a limit or an aperture; TODO_BODY, the body
-// by body_near and those checks; TODO_ALL, the whole element by the general
-// maps.  With the last two p is as it was.  fl: the header's flags.  TIME: the instance carries the
-// particle time.
+// track1 through a record by its near-axis form.  What is left to do
+// (track1_finish): TODO_NOTHING; TODO_EXIT, the checks after the body, where
+// the particle may be past a limit or an aperture; TODO_BODY, the body and
+// those checks; TODO_ALL, the whole element by the general maps.  With the
+// last two p is as it was.  fl: the header's flags.  TIME: the instance
+// carries the particle time.
 // With then (the record has F_THEN_DRIFT) its drift record follows in the same
 // call, without the loads, tests and the vote of an element of its own (1M
 // particles x 2 turns 18.1 -> 16.9 ms, 10,000 x 16 turns 8.45 -> 7.35);
@@ -467,7 +491,7 @@ __device__ __forceinline__ int track1_near(Part& p, const double* rec, int32_t f
   if ((fl & F_AP_ENTRANCE) && G.ap_on && !inside_aperture(p, ap, fl)) return TODO_ALL;
   if (kind == K_DRIFT) {
     drift_record_near<TIME>(p, q - HDR_DW, G, m.a, m.r_pc);
-  } else {
+  } else if (kind != K_MARKER) {
     const qp::Q t0 = time_of(p);
     const double z0 = p.z;
     double dt_ref;
@@ -482,9 +506,9 @@ __device__ __forceinline__ int track1_near(Part& p, const double* rec, int32_t f
       quad_steps<NoKicks>(p, M, dz_low, h, q);
       dt_ref = q[Q_DTREF];
     } else {
-      if ((fl & F_MISALIGN) || h->poles != 4) return TODO_BODY;
+      if ((fl & F_MISALIGN) || !PlainKicks::holds(h->poles)) return TODO_BODY;
       Saved start(p);
-      if (!thick_steps<DenseKicks<2, 2>>(p, h, q, G.mal, m.a, m.r_pc)) {
+      if (!thick_steps<PlainKicks>(p, h, q, G.mal, m.a, m.r_pc)) {
         start.restore(p);
         return TODO_ALL;
       }

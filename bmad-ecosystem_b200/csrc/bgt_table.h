@@ -85,8 +85,8 @@ enum Flag : int32_t {
   // F_AP_MOM_ELL: the ecollimator's elliptical pairs
   F_AP_MOMENTUM = 1 << 28,
   F_AP_MOM_ELL = 1 << 29,
-  // the record has a near-axis form (bgt_near.cuh): a drift; a plain bend; a
-  // quadrupole or thick multipole with magnetic multipoles up to order 7 and
+  // the record has a near-axis form (bgt_near.cuh): a marker or drift; a plain
+  // bend; a quadrupole or thick multipole with magnetic multipoles up to order 7 and
   // offsets and roll at most; lab-frame apertures without momentum limits
   F_NEAR = 1 << 30,
   // the record has a near-axis form other than a drift's, and the next one of

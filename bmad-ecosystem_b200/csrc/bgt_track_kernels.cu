@@ -11,8 +11,8 @@
 //     128 x (3, 4, 5), 256 x (2, 3) -- 128 x 3 (168 registers, no spills) for
 //     small long-lived sets where one particle's turn latency sets the time.
 // A group has one register cap: the out-of-line functions of a compilation
-// unit (track1_general) are compiled once, for the smallest cap of the kernels
-// that call them, and at the 64 of 256 x 4 they spill 3 KB a thread.
+// unit (the rare edges and frames, correctly rounded functions' slow paths) are
+// compiled once, for the smallest cap of the kernels that call them.
 #include "bgt_kernel.cuh"
 
 #ifndef BGT_KERNEL_GROUP
