@@ -7,6 +7,8 @@ memory instead of shared memory (frees shared memory for more resident CTAs
 when tables are large), and, for lossy workloads, the compaction interval.  Each
 candidate tracks a sample of the real bunch for a few turns on the device
 (CUDA events on the launching stream); the fastest per particle.turn wins.
+Shapes with table_mode 0 are fitted to the call by the library (bgt.h), here
+as in later calls, so two of them may be the same launch on a small sample.
 Results are cached per (table bytes, lattice name, particle count) in memory
 and, when a path is given, in a JSON file.
 """

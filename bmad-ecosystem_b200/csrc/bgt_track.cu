@@ -19,6 +19,7 @@
 #include "../../include/bgt.h"
 #include "bgt_compile.h"
 #include "bgt_kernel.cuh"
+#include "bgt_launch_fit.h"
 
 // ===========================================================================
 // Handle and C ABI
@@ -234,40 +235,12 @@ static uint64_t wait_ns_of(const bgt_tuning& t) {
   return t.wait_limit_us > 0 ? (uint64_t)t.wait_limit_us * 1000ull : 2000000000ull;
 }
 
-// A tuning fitted to a call: the shape and table placement to launch.
-// n_tiles(block): the tiles of `block` particles that the call makes.
-//
-// * 256-thread tiles become 128-thread ones with the same register cap while
-//   all of them are resident at once: a CTA's warps share an SM, so few large
-//   tiles leave SMs idle or uneven.  Measured on B200, 256 x 2 against
-//   128 x 4: 40,000 particles x 4 turns of the FODO ring 2.70 / 2.40 ms,
-//   10,000 2.25 / 2.07 ms, one turn of 8,064 probes on four error rings
-//   2.08 / 1.90 ms; from one full wave on they are equal.
-// * table_mode 0 stages the table in shared memory only if that leaves room
-//   for the CTAs the launch can use per SM; a staged 150 KB table (error
-//   rings) holds one.  Staged against global, 128 x 4, one turn on error
-//   rings: 60,000 particles (4 CTAs per SM wanted) 7.39 / 3.31 ms, 32,000 (2)
-//   3.75 / 2.33 ms, 16,000 (1) 1.92 / 2.15 ms.
 template <class NTiles>
-static bgt_tuning fit_tuning(bgt_tuning t, size_t table_dw, int num_sms, bool rare, const NTiles& n_tiles) {
-  const bool compact = t.compact_every > 0;
-  // whether a staged table leaves every CTA resident that the launch can use
-  // (228 KB of shared memory per SM, 1 KB of it per CTA reserved)
-  auto staged_fits = [&](int block, int per_sm) {
-    const size_t smem = smem_bytes(table_dw, block, compact, false, rare);
-    const int64_t wanted = std::min<int64_t>(per_sm, (n_tiles(block) + num_sms - 1) / num_sms);
-    return smem <= SMEM_LIMIT && (int64_t)((228 * 1024) / (smem + 1024)) >= wanted;
-  };
-  const int mode = t.table_mode >= 2 ? t.table_mode - 1 : 0;  // the kernels' TMODE
-  if (t.threads_per_block == 256 && n_tiles(256) < (int64_t)t.blocks_per_sm * num_sms &&
-      find_track_kernel(128, 2 * t.blocks_per_sm, mode, rare) && (mode != 0 || staged_fits(128, 2 * t.blocks_per_sm))) {
-    t.threads_per_block = 128;
-    t.blocks_per_sm *= 2;
-  }
-  if (t.table_mode == 0 && !staged_fits(t.threads_per_block, t.blocks_per_sm) &&
-      find_track_kernel(t.threads_per_block, t.blocks_per_sm, 1, rare))
-    t.table_mode = 2;
-  return t;
+static bgt_tuning fit_tuning(const bgt_tuning& t, size_t table_dw, int num_sms, bool rare, const NTiles& n_tiles) {
+  return bgt::fit_tuning(
+      t, num_sms, SMEM_LIMIT, n_tiles,
+      [&](int block) { return smem_bytes(table_dw, block, t.compact_every > 0, false, rare); },
+      [&](int block, int per_sm, int tmode) { return find_track_kernel(block, per_sm, tmode, rare) != nullptr; });
 }
 
 // The kernel instance for a tuning and a shared-memory need, with the

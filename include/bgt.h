@@ -171,7 +171,11 @@ typedef struct bgt_species {
   int32_t absolute_time_ref_shift; /* bmad_com%absolute_time_ref_shift (default 1) */
 } bgt_species;
 
-/* Launch tiles chosen by the autotuner (0 = let the library choose). */
+/* Launch tiles chosen by the autotuner (0 = let the library choose).  With
+ * table_mode 0 the library fits the launch to the call: the table's placement,
+ * and 128-thread CTAs, twice as many per SM, in place of 256-thread ones while
+ * one wave holds them all.  With table_mode 1, 2 or 3 the shape is launched as
+ * given.  Results do not depend on it. */
 typedef struct bgt_tuning {
   int32_t threads_per_block; /* particles per CTA */
   int32_t blocks_per_sm;     /* resident CTAs per SM for the persistent grid */
