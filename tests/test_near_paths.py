@@ -52,5 +52,9 @@ def test_every_way_through_a_record(checker, seed):
             # the exact low-energy correction is the general map's: |pz| above
             # 0.054, two thirds of a quarter of the particles
             assert way > 0.79 * total, (name, kernel)
+        elif form.startswith("bend"):
+            # its 12 rounding tests, each of which may fail for 1 in 1000
+            # arguments (test_near_maps.py), leave a particle to the general map
+            assert way > 0.988 * total, (name, kernel)
         else:
             assert way == total, (name, kernel)
