@@ -1522,6 +1522,17 @@ static int train_batch(bgt_mlp* m, const bf16* X, const float* label, int32_t ba
   return 0;
 }
 
+// whether p is a float array in the memory of the handle's device
+static bool own_floats(const bgt_mlp* m, const float* p) {
+  cudaPointerAttributes a{};
+  if ((uintptr_t)p % sizeof(float) != 0) return false;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == m->device;
+}
+
 static int check_batch(bgt_mlp* m, const uint16_t* d_x, const float* d_label, int32_t batch) {
   if (!m || !d_x || !d_label) return BGT_EINVAL;
   if (batch <= 0 || batch % 128 || batch > m->max_batch)
@@ -1551,8 +1562,13 @@ int bgt_mlp_gradients(bgt_mlp* m, const uint16_t* d_x, const float* d_label, int
   if (rc) return rc;
   MCU(m, cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
-  rc = train_batch(m, reinterpret_cast<const bf16*>(d_x), d_label, batch, d_grad ? d_grad : m->grads, AdamStep{}, st);
+  // the kernel writes a caller's array on the handle's device itself; any
+  // other (not a float's alignment, another device's, host memory) is copied to
+  const bool direct = d_grad && own_floats(m, d_grad);
+  rc = train_batch(m, reinterpret_cast<const bf16*>(d_x), d_label, batch, direct ? d_grad : m->grads, AdamStep{}, st);
   if (rc) return rc;
+  if (d_grad && !direct)
+    MCU(m, cudaMemcpyAsync(d_grad, m->grads, N_PARAMS * sizeof(float), cudaMemcpyDeviceToDevice, st));
   if (loss) {
     MCU(m, cudaMemcpyAsync(loss, m->scalars, sizeof(float), cudaMemcpyDeviceToHost, st));
     MCU(m, cudaStreamSynchronize(st));
