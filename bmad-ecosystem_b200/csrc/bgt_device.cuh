@@ -383,6 +383,13 @@ __device__ __forceinline__ void check_aperture(Part& p, const double* ap, const 
 __device__ __forceinline__ void drift_memo(const Part& p, const Glob& G, DriftMemo& m) {
   if (p.pz != m.pz) {
     double delta = p.pz;
+#ifdef __CUDACC__
+    // keeps the quotients and the root behind the test: pz does not change in
+    // the loop of near-axis forms, and the compiler would otherwise evaluate
+    // them at every entry of that loop (five quotients, a root and 60 FP64
+    // instructions at each magnet of an error ring)
+    asm volatile("" : "+d"(delta));
+#endif
     double rel_pc = 1 + delta;
     m.a = sqrt_one((G.mc2sq * (2 * delta + delta * delta)) / (sq(G.p0c * rel_pc) + G.mc2sq));
     m.r_pc = 1.0 / rel_pc;

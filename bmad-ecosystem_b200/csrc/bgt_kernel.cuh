@@ -750,7 +750,7 @@ __device__ __forceinline__ int track1_finish(Part& p, const double* rec, const d
       if (RARE) element_exit_time(p, t0, z0, q[h->kind == K_QUAD ? Q_DTREF : TM_DTREF], G);
     }
     if (orbit_too_large(p, G)) return 0;
-    if ((fl & F_AP_EXIT) && G.ap_on) aperture_limits(p, ap, fl, p.x, p.y);
+    if ((fl & F_AP_EXIT) && G.ap_on && !inside_aperture(p, ap, fl)) aperture_limits(p, ap, fl, p.x, p.y);
     if (p.state != ALIVE) return 0;
     if (!then || !(abs_hi(p.px) < m.near_p && abs_hi(p.py) < m.near_p)) return 1;
     drift_record_near<RARE>(p, then, G, m.a, m.r_pc);
@@ -811,7 +811,7 @@ void track1_general(GeneralCall* io, const double* rec, QMemo qm, int) {
 // local memory writes through to L2: 606,208 particles x 16 elements took
 // 0.38 ms of markers, 0.46 of kickers, 0.81 of rbends, and 0.43 of drifts for
 // particles outside the near-axis region.  Side by side the register sets are
-// separate: 0.07, 0.13, 0.58 and 0.16 ms (with the general maps alone, before
+// separate: 0.07, 0.13, 0.55 and 0.16 ms (with the general maps alone, before
 // there were near-axis forms: 0.08, 0.20, 0.57, 0.14).
 //
 // The warp leaves the general loop at a record whose near-axis form pays for
