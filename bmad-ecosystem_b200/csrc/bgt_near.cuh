@@ -13,8 +13,8 @@
 // SM.  Through the general maps alone a warp takes 319,000 instructions per
 // turn of the 770-element ring, 140,000 of them FP64, at 44 % FP64 pipe: 17.7
 // ns per particle and turn (1M particles, 256 x 2).  With the near-axis
-// forms: ~155,000, 76,000 FP64, 8.4 ns; one warp alone on its scheduler
-// (10,000 particles) 0.46 ms per turn instead of 1.13.
+// forms: 153,000, 75,000 FP64, 7.6 ns; one warp alone on its scheduler
+// (10,000 particles) 0.41 ms per turn instead of 1.13.
 #pragma once
 
 namespace bgt {
